@@ -75,6 +75,54 @@ struct Symbolic {
 };
 Symbolic analyse(const Grid &g, const YPattern &y, std::string *why);
 
+// The schedule of k_lu_cluster (cluster.cuh), one part per CTA of the cluster:
+// part c = ints off[c] .. off[c + 1] of blob (multiples of four).  Steps
+// (pivots, in elimination order) 0 .. t0-1 run level by level on the whole
+// cluster; steps t0 .. td-1 are the segment that CTA 0 keeps in its shared
+// memory; steps td .. n-1 are the tail, a dense trailing block (every step's
+// row is full) that is factored right-looking in the shared memory of
+// tail_ctas CTAs, block column c on CTA c % tail_ctas.  A part holds, in order,
+//   nf1 forward levels, the gather of the cluster's updates into the segment
+//   and the tail, nfs forward levels of the segment, the gather of the
+//   segment's updates into the tail (8 ints each: pivots, entries, where their
+//   records start, cfg), nbs backward levels of the segment and nb1 of the
+//   cluster (4 ints each: rows, where their records start, cfg);
+//   records of four ints: pivot j / entry position p / row j, first and end
+//   index of its list, and for a pivot whether this CTA stores it, for an
+//   entry where its pivot's inverse is (cluster: the pivot's index in the
+//   CTA's level, segment: j), for an entry of the gather into the tail its
+//   block row and column there (row << 16 | column);
+//   lists of pairs: (position, step) for pivots, (position of L(j,k),
+//   position of L(i,k)) for entries, (position, column) for rows, packed in
+//   one int (second << 16 | first) when every position fits 16 bits, else two.
+// cfg: bits 0-2 / 3-5 log2 of the lanes per pivot (row) / entry, bits 6 / 7:
+// lanes counted in quads (a 2x2 block on four lanes), bits 8-10 / 11-13 log2 of
+// the warps that the pivots (rows) / entries are dealt to, bit 14: the entries
+// fit one pass of those warps, bits 16-: warps by which the entries are
+// rotated past the pivots.
+constexpr int kClusterThreads = 512;
+constexpr int kTailMin = 16, kTailMax = 96, kTailMax32 = 64;  // orders of a tail (on one CTA: kTailMax32)
+struct ClusterSchedule {
+    std::vector<int> blob, off;
+    int ctas = 0, t0 = 0, td = 0, tail_ctas = 1, nf1 = 0, nfs = 0, nbs = 0, nb1 = 0;
+    int packed = 0;      // lists of one int a pair
+    int max_ints = 0;    // longest part
+    int max_pivots = 0;  // most pivots of a CTA in one cluster level
+    // dynamic shared memory of a launch: pivot inverses of a level, the
+    // segment's blocks, the vectors of steps t0 .. n-1, the tail, the schedule
+    // (0: it stays in global memory)
+    size_t inv_bytes = 0, seg_bytes = 0, vec_bytes = 0, tail_bytes = 0, sched_bytes = 0;
+};
+ClusterSchedule cluster_schedule(const Symbolic &S, int ctas, bool fp64, size_t smem_limit);
+// Blocks of shared memory of the tail of order m on `ctas` CTAs: its columns
+// and the right-hand side, the inverses, two copies of the pivot column and,
+// on CTA 0, the strict upper triangle for the backward substitution (one CTA
+// has that in its columns, and a second copy of them before the updates).
+inline size_t tail_blocks(int m, int ctas) {
+    const size_t cols = ((size_t)m + 1 + ctas - 1) / ctas * m;
+    return ctas == 1 ? 2 * cols + m : cols + m + 2 * (size_t)m + (size_t)m * (m - 1) / 2;
+}
+
 // Ordering used by analyse(): minimum degree on the bus graph, then the
 // perfect elimination order of its filled graph with the shortest elimination
 // tree (reduce_height: same fill, fewer levels).

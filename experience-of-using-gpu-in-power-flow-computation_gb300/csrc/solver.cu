@@ -13,8 +13,8 @@
 // mismatch, test) followed by a conditional WHILE node whose body is one Newton
 // iteration; the test kernel sets the loop condition on the device, so a solve
 // is one graph launch and one host synchronisation.  The LU and substitutions
-// run one kernel per elimination level, or for small grids every level in one
-// single-block kernel (k_lu_fused).
+// run in one launch of a thread-block cluster (k_lu_cluster), or one kernel per
+// elimination level, or every level in one single-block kernel (k_lu_fused).
 //
 // Jacobian layout: 2x2 blocks per non-slack bus ([dP/dth dP/dV; dQ/dth dQ/dV]),
 // with a Q row and V column for every non-slack bus.  Buses that are PV (not at
@@ -646,12 +646,19 @@ __global__ void k_bsolve(Dev d, int beg, int cnt, int guard) {
 // launches would cost more than their work.  A singular pivot stops it at the
 // next level boundary, as the per-level launches stop (guard).
 constexpr int kFusedThreads = 512;
-// Largest Jacobian block order that takes k_lu_fused by default.  Measured on
-// single solves (ms per solve, per-level launches -> k_lu_fused): FP32 57
-// buses 0.99 -> 0.57, 118 0.79 -> 0.46, 236 5.7 -> 3.5, 472 18.5 -> 13.3, 944
-// 19.8 -> 23.3, 1,888 1.35 -> 1.73; FP64 57 1.99 -> 1.76, 118 1.53 -> 1.40,
-// 236 16.9 -> 19.6 (one SM's FP64 pipe is too small for more).
+// Largest Jacobian block order that takes k_lu_fused rather than a launch per
+// level where k_lu_cluster does not run: FP32 with reactive limits (the limit
+// check looks at the size of the Newton step, whose FP32 rounding k_lu_fused's
+// order of sums keeps on the FP64 switch path of the 118-bus golden cases),
+// and GPUs without clusters of 8.  Measured on single solves (ms per solve,
+// per-level launches -> k_lu_fused): FP32 57 buses 0.99 -> 0.57, 118 0.79 ->
+// 0.46, 236 5.7 -> 3.5, 472 18.5 -> 13.3, 944 19.8 -> 23.3, 1,888 1.35 -> 1.73;
+// FP64 57 1.99 -> 1.76, 118 1.53 -> 1.40, 236 16.9 -> 19.6 (one SM's FP64 pipe
+// is too small for more).
 constexpr int kFusedMaxN32 = 600, kFusedMaxN64 = 150;
+// Largest factor (off-diagonal blocks a triangle) whose FP64 solve takes the
+// persistent form by default (see gbpf_solver::build).
+constexpr int kOneMaxBlocks = 300;
 template <typename TJ>
 __global__ void __launch_bounds__(kFusedThreads, 1) k_lu_fused(Dev d, int guard) {
     __shared__ int s_stop;
@@ -672,6 +679,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_lu_fused(Dev d, int guard)
         __syncthreads();
     }
 }
+
+#include "cluster.cuh"
 
 // attOlim / attVlim: theta += dx_theta, V += dx_V on active rows; max|dx|.
 __global__ void k_update(Dev d, int guard) {
@@ -776,6 +785,7 @@ struct gbpf_solver {
         if (pexec) cudaGraphExecDestroy(pexec);
         if (pgraph) cudaGraphDestroy(pgraph);
         if (one) gbpf::one_free(one);
+        if (cl_mem) cudaFree(cl_mem);
         if (flat_on) cudaFree(flat_on);
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
@@ -811,13 +821,42 @@ struct gbpf_solver {
     }
     // Levels whose steps carry more gather work than a warp should take on
     // alone (level_heavy) run one block per step.
-    // lu_fused: every level in one k_lu_fused launch (made by launch_forward;
-    // launch_backward then launches nothing)
+    // lu_fused: 1 = every level in one k_lu_fused launch, 2 = in one
+    // k_lu_cluster launch (made by launch_forward; launch_backward then
+    // launches nothing)
     int lu_fused = 0;
+    int cl_ctas = 0;  // CTAs of k_lu_cluster's cluster, 0: not available
+    ClArgs cl_args{};
+    size_t cl_smem = 0;
+    void *cl_mem = nullptr;  // the schedule
+    gbpf_status plan_cluster();
+    cudaLaunchConfig_t cluster_config(int ctas, size_t smem, cudaLaunchAttribute *at) const {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(ctas);
+        cfg.blockDim = dim3(kClT);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        at->id = cudaLaunchAttributeClusterDimension;
+        at->val.clusterDim.x = ctas;
+        at->val.clusterDim.y = at->val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cfg;
+    }
+    int lu_mode(int mode) const {
+        if (mode == 0 && cl_ctas && !(d.fp32 && opt.lim_inj_reat && S.n <= kFusedMaxN32)) return 2;
+        return mode == 2 || (mode == 0 && S.n <= (d.fp32 ? kFusedMaxN32 : kFusedMaxN64));
+    }
     template <typename TJ> void launch_forward_t(int guard) {
         const int T = 256, W = T / 32;
-        if (lu_fused) {
+        if (lu_fused == 1) {
             k_lu_fused<TJ><<<1, kFusedThreads, 0, stream>>>(d, guard);
+            return;
+        }
+        if (lu_fused == 2) {
+            cudaLaunchAttribute at[1];
+            const cudaLaunchConfig_t cfg = cluster_config(cl_ctas, cl_smem, at);
+            (void)cudaLaunchKernelEx(&cfg, k_lu_cluster<TJ>, d, cl_args, guard);
             return;
         }
         for (int l = 0; l < nfl(); l++) {
@@ -890,6 +929,8 @@ struct gbpf_solver {
 
     gbpf_status build(const Grid &grid, const gbpf_options &o, int dev);
     gbpf_status build_graph();
+    gbpf_status ensure_graph();
+    bool lu_planned = false;
     gbpf_status build_persistent();
     gbpf_status record_persistent();
     gbpf_status run(gbpf_result *r);
@@ -1096,30 +1137,73 @@ gbpf_status gbpf_solver::build(const Grid &grid, const gbpf_options &o, int dev)
     CK(cudaStreamSynchronize(stream));
     setup_ms[0] += ms_since(tp);
     tp = clk::now();
-    lu_fused = !d.dense_rule && n <= (d.fp32 ? kFusedMaxN32 : kFusedMaxN64);
-    gbpf_status st = build_graph();
+    gbpf_status st = GBPF_OK;
     // the persistent form where the grid's state fits one block's shared
-    // memory (metodo = esparso); it is the default in FP64.  The FP32-LU form
-    // keeps the graph by default: its block kernel's one-pass FP32 levels
+    // memory (metodo = esparso).  It is the default in FP64 for factors of at
+    // most kOneMaxBlocks off-diagonal blocks a triangle, the size up to which
+    // one SM's FP64 pipe keeps up with the cluster's.  Measured ms per FP64
+    // solve, persistent / graph with k_lu_cluster (blocks): ieee14 0.08 / 0.16
+    // (21), ieee118 0.215 / 0.256 (253), a filled 57-bus grid 0.291 / 0.293
+    // (221), 80-bus 0.369 / 0.346 (323), ieee118x2 0.336 / 0.318 (533), filled
+    // 118-bus 0.545 / 0.445 (568), 236-bus 1.92 / 0.71 (1,736), 1,888-bus 1.48 /
+    // 0.60 (4,237), filled 472-bus 9.55 / 1.46 (5,422).  The FP32-LU form keeps
+    // the graph by default: its block kernel's one-pass FP32 levels
     // round the Newton step differently, and on a 118-bus grid with reactive
     // limits that kept every step above the limit trigger's 10 tol until
     // convergence, so no PV bus switched (the graph form's FP32 steps follow
     // the FP64 switch path there).
-    if (st == GBPF_OK && !d.dense_rule) {
+    // Each form is built when it is first asked for.
+    if (!d.dense_rule && !d.fp32 && nup <= kOneMaxBlocks) {
         const std::string keep = gbpf::last_error();
-        if (build_persistent() == GBPF_OK) form = d.fp32 ? GBPF_FORM_GRAPH : GBPF_FORM_PERSISTENT;
+        if (build_persistent() == GBPF_OK) form = GBPF_FORM_PERSISTENT;
         else set_error(keep);
     }
+    if (form == GBPF_FORM_GRAPH) st = ensure_graph();
     setup_ms[4] = ms_since(tp);
     return st;
+}
+
+// The schedule of k_lu_cluster on the device, and the cluster it runs on: 16
+// CTAs where the GPU schedules such clusters, else 8 (1 where the whole factor
+// fits one CTA's shared memory).
+gbpf_status gbpf_solver::plan_cluster() {
+    int optin = 0;
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    const void *fn = d.fp32 ? (const void *)k_lu_cluster<float> : (const void *)k_lu_cluster<double>;
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (int ctas : {16, 8}) {
+        const gbpf::ClusterSchedule cl = gbpf::cluster_schedule(S, ctas, !d.fp32, (size_t)optin - 1024);
+        if (!cl.ctas) continue;
+        const size_t at_seg = cl.inv_bytes, at_vec = at_seg + cl.seg_bytes, at_tail = at_vec + cl.vec_bytes,
+                     at_sched = at_tail + cl.tail_bytes, sm = at_sched + cl.sched_bytes;
+        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = cluster_config(cl.ctas, sm, at);
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, fn, &cfg) != cudaSuccess) { (void)cudaGetLastError(); fit = 0; }
+        if (fit < 1) continue;
+        CK(cudaMalloc(&cl_mem, 4 * (cl.blob.size() + cl.off.size())));
+        CK(cudaMemcpy(cl_mem, cl.blob.data(), 4 * cl.blob.size(), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy((int *)cl_mem + cl.blob.size(), cl.off.data(), 4 * cl.off.size(), cudaMemcpyHostToDevice));
+        cl_args = {(const int *)cl_mem, (const int *)cl_mem + cl.blob.size(), cl.t0, cl.td, cl.tail_ctas,
+                   S.up_ptr[cl.t0], S.up_ptr[cl.td], cl.nf1, cl.nfs, cl.nbs, cl.nb1, cl.packed, cl.sched_bytes > 0,
+                   (int)at_seg, (int)at_vec, (int)at_tail, (int)at_sched};
+        cl_smem = sm;
+        cl_ctas = cl.ctas;
+        break;
+    }
+    return GBPF_OK;
 }
 
 // The persistent form's graph: one launch of the batch's block kernel that
 // runs the whole Newton loop on this solver's arrays, then the branch flows.
 gbpf_status gbpf_solver::build_persistent() {
-    gbpf_status st = gbpf::one_create(g, opt, device, &one);
+    if (pexec) return GBPF_OK;
+    if (d.dense_rule) return GBPF_E_UNSUPPORTED;
+    gbpf_status st = GBPF_OK;
+    if (!one) st = gbpf::one_create(g, opt, device, &one);
     if (st != GBPF_OK) return st;
-    CK(cudaMalloc(&flat_on, sizeof(int)));
+    if (!flat_on) CK(cudaMalloc(&flat_on, sizeof(int)));
     CK(cudaMemcpy(flat_on, &flat_on_h, sizeof(int), cudaMemcpyHostToDevice));
     return record_persistent();
 }
@@ -1151,6 +1235,19 @@ gbpf_status gbpf_solver::record_persistent() {
     pgraph = gr;
     CK(cudaGraphInstantiate(&pexec, pgraph, 0));
     return GBPF_OK;
+}
+
+// The graph form's LU launch and graph, when something first needs them.
+gbpf_status gbpf_solver::ensure_graph() {
+    if (exec) return GBPF_OK;
+    CK(cudaSetDevice(device));
+    if (!d.dense_rule && !lu_planned) {
+        const gbpf_status st = plan_cluster();
+        if (st != GBPF_OK) return st;
+        lu_planned = true;
+        lu_fused = lu_mode(0);
+    }
+    return build_graph();
 }
 
 gbpf_status gbpf_solver::build_graph() {
@@ -1268,14 +1365,15 @@ extern "C" gbpf_status gbpf_solver_set_start(gbpf_solver *s, const double *V0, c
     CK(cudaSetDevice(s->device));
     if (V0) CK(cudaMemcpyAsync(s->d.V0, V0, b, cudaMemcpyHostToDevice, s->stream));
     if (theta0) CK(cudaMemcpyAsync(s->d.th0, theta0, b, cudaMemcpyHostToDevice, s->stream));
-    if ((V0 || theta0) && s->flat_on) {
+    if (V0 || theta0) {
         // the persistent form takes iteration 0 from the topology's shared copy
         // only while the start is the grid's own
         const bool own = (!V0 || std::equal(V0, V0 + s->g.nB, s->g.V0.begin())) &&
                          (!theta0 || std::equal(theta0, theta0 + s->g.nB, s->g.theta0.begin()));
         if ((int)own != s->flat_on_h) {
             s->flat_on_h = own;
-            CK(cudaMemcpyAsync(s->flat_on, &s->flat_on_h, sizeof(int), cudaMemcpyHostToDevice, s->stream));
+            if (s->flat_on)
+                CK(cudaMemcpyAsync(s->flat_on, &s->flat_on_h, sizeof(int), cudaMemcpyHostToDevice, s->stream));
         }
     }
     if (Pliq) CK(cudaMemcpyAsync(s->d.Pliq, Pliq, b, cudaMemcpyHostToDevice, s->stream));
@@ -1359,7 +1457,9 @@ extern "C" gbpf_status gbpf_solver_set_lu_launch(gbpf_solver *s, int mode) {
     if (s->d.dense_rule) { set_error("metodo = denso has no level-scheduled LU"); return GBPF_E_ARG; }
     CK(cudaSetDevice(s->device));
     CK(cudaStreamSynchronize(s->stream));
-    const int fused = mode == 2 || (mode == 0 && s->S.n <= (s->d.fp32 ? kFusedMaxN32 : kFusedMaxN64));
+    gbpf_status st = s->ensure_graph();
+    if (st != GBPF_OK) return st;
+    const int fused = s->lu_mode(mode);
     const int split = mode == 3 ? 0 : 1;
     if (fused == s->lu_fused && split == s->split_heavy) return GBPF_OK;
     s->lu_fused = fused;
@@ -1371,26 +1471,30 @@ extern "C" gbpf_status gbpf_solver_set_lu_launch(gbpf_solver *s, int mode) {
 
 extern "C" gbpf_status gbpf_solver_set_form(gbpf_solver *s, int form) {
     ARGCHECK(s && (form == GBPF_FORM_GRAPH || form == GBPF_FORM_PERSISTENT));
-    if (form == GBPF_FORM_PERSISTENT && !s->pexec) {
+    CK(cudaSetDevice(s->device));
+    CK(cudaStreamSynchronize(s->stream));
+    if (form == GBPF_FORM_PERSISTENT && s->build_persistent() != GBPF_OK) {
         set_error("this grid has no persistent form (metodo = denso, or its state does not fit one block's shared "
                   "memory)");
         return GBPF_E_UNSUPPORTED;
     }
-    CK(cudaSetDevice(s->device));
-    CK(cudaStreamSynchronize(s->stream));
+    if (form == GBPF_FORM_GRAPH) {
+        const gbpf_status st = s->ensure_graph();
+        if (st != GBPF_OK) return st;
+    }
     s->form = form;
     return GBPF_OK;
 }
 
 extern "C" gbpf_status gbpf_solver_set_plan(gbpf_solver *s, int lu1, int narrow, int quad, int out[3]) {
     ARGCHECK(s);
-    if (!s->one) {
+    CK(cudaSetDevice(s->device));
+    CK(cudaStreamSynchronize(s->stream));
+    if (s->build_persistent() != GBPF_OK) {
         set_error("this grid has no persistent form (metodo = denso, or its state does not fit one block's shared "
                   "memory)");
         return GBPF_E_UNSUPPORTED;
     }
-    CK(cudaSetDevice(s->device));
-    CK(cudaStreamSynchronize(s->stream));
     gbpf_status st = gbpf::one_set_plan(s->one, lu1, narrow, quad, out);
     if (st != GBPF_OK) return st;
     return (lu1 >= 0 || narrow >= 0 || quad >= 0) ? s->record_persistent() : GBPF_OK;
@@ -1410,6 +1514,8 @@ extern "C" gbpf_status gbpf_solver_get_form(const gbpf_solver *s, int out[3]) {
 
 extern "C" gbpf_status gbpf_solver_info(const gbpf_solver *s, long long info[8]) {
     ARGCHECK(s && info);
+    const gbpf_status st = const_cast<gbpf_solver *>(s)->ensure_graph();  // its launches are reported
+    if (st != GBPF_OK) return st;
     info[0] = s->g.nB;
     info[1] = s->S.n;
     info[2] = s->S.nup;
@@ -1449,6 +1555,8 @@ extern "C" gbpf_status gbpf_solver_setup_times(const gbpf_solver *s, double ms[5
 extern "C" gbpf_status gbpf_solver_profile(gbpf_solver *s, int repeats, double ms[4], long long bytes[4]) {
     ARGCHECK(s && ms && bytes && repeats > 0);
     CK(cudaSetDevice(s->device));
+    const gbpf_status st = s->ensure_graph();
+    if (st != GBPF_OK) return st;
     const Symbolic &S = s->S;
     const int T = 256, nq = S.n + 2 * S.nup;
     const bool dense = s->d.dense_rule;
@@ -1606,7 +1714,8 @@ extern "C" gbpf_status gbpf_eval_jacobian(gbpf_solver *s, const double *V, const
 extern "C" gbpf_status gbpf_newton_step(gbpf_solver *s, const double *V, const double *theta,
                                         const int *limQ, const double *gref, double *dx) {
     ARGCHECK(s && V && theta && gref && dx);
-    gbpf_status st = load_state(s, V, theta, limQ);
+    gbpf_status st = s->ensure_graph();
+    if (st == GBPF_OK) st = load_state(s, V, theta, limQ);
     if (st != GBPF_OK) return st;
     const Symbolic &S = s->S;
     std::vector<int> pn, qn;
@@ -1646,6 +1755,10 @@ extern "C" gbpf_status gbpf_newton_step(gbpf_solver *s, const double *V, const d
 extern "C" gbpf_status gbpf_solve_traced(gbpf_solver *s, gbpf_result *r, gbpf_trace_fn fn, void *user) {
     ARGCHECK(s && fn);
     CK(cudaSetDevice(s->device));
+    {
+        const gbpf_status sg = s->ensure_graph();
+        if (sg != GBPF_OK) return sg;
+    }
     const Grid &g = s->g;
     const Symbolic &S = s->S;
     const Dev &d = s->d;

@@ -304,15 +304,18 @@ gbpf_status gbpf_solve_traced(gbpf_solver *s, gbpf_result *r, gbpf_trace_fn fn, 
  * each); 3 = as 1 but those levels as one kernel of one block per step (its
  * entries walked by that block); 2 = every level in one single-block kernel
  * with a barrier between levels (k_lu_fused: same per-step arithmetic, no
- * per-level launch); 0 = 2 up to 600 block rows (buses - 1) in the FP32-LU
- * form and 150 in FP64, else 1 (the default).  1 and 3 give the same factor.
- * Rebuilds the graph.  Not for metodo = denso. */
+ * per-level launch); 0 = the default: every level in one launch of a
+ * thread-block cluster (k_lu_cluster), but for the FP32-LU form with reactive
+ * limits up to 600 block rows (buses - 1), which takes 2.  1 and 3 give the
+ * same factor.  Rebuilds the graph.  Not for metodo = denso. */
 gbpf_status gbpf_solver_set_lu_launch(gbpf_solver *s, int mode);
 
 /* The form gbpf_solve runs (gbpf_form).  gbpf_solver_create picks
- * GBPF_FORM_PERSISTENT for metodo = esparso in FP64 wherever the grid's state
- * fits one block's shared memory (up to ~1,900 buses) and GBPF_FORM_GRAPH
- * otherwise (the FP32-LU form may still be set to PERSISTENT); in FP64 the
+ * GBPF_FORM_PERSISTENT for metodo = esparso in FP64 on small grids (a factor
+ * of at most 300 off-diagonal blocks a triangle, about 120 buses) and
+ * GBPF_FORM_GRAPH otherwise; PERSISTENT may be set on any grid whose state
+ * fits one block's shared memory (up to ~1,900 buses in FP64), the FP32-LU
+ * form included; in FP64 the
  * same iterations, switch events, |V|, theta, history and flows come out of
  * both.  set: GBPF_E_UNSUPPORTED when the grid cannot run
  * PERSISTENT.  get: out[0] = the form, out[1] = kernel launches per solve of

@@ -1,0 +1,85 @@
+"""GPU: the LU and substitutions in one thread-block cluster (k_lu_cluster, the
+graph form's default) against one kernel per elimination level
+(gbpf_solver_set_lu_launch mode 1), over its schedules: the whole factor in one
+CTA (small grids), cluster levels with a segment (chains of copies), with a
+dense tail just over its least order, of 78 and with 43 levels before it, and
+without either."""
+import numpy as np
+import pytest
+
+from conftest import ieee_cases, ieee_path
+
+pytestmark = pytest.mark.gpu
+
+
+def grid_of(gb, name):
+    if name.startswith("gen"):
+        return gb.generate(4, 11, nbus=int(name[3:]))
+    if name.startswith("ieee"):
+        return gb.read_grid(ieee_path(next(c for c in ieee_cases() if c["cdf"] == name + ".cdf")))
+    import bench
+
+    return gb.read_grid(bench.grid_file(name))
+
+
+# Two factorisations of one Jacobian differ by rounding only, and Newton ends on the same solution: in FP64 the last
+# step's rounding is eps kappa |dx| with kappa <= 1e5 and |dx| <= 1e-2, below 1e-12 with room for the tiled grids'
+# larger angles: 1e-11.  In FP32 the last step before max|g| <= 1e-10 is at most about 1e-5 and its relative error
+# eps32 kappa <= 6e-3: 1e-7.
+@pytest.mark.parametrize("precision,tol,atol", [("PREC_FP64", 1e-8, 1e-11), ("PREC_FP32_IR", 1e-10, 1e-7)])
+@pytest.mark.parametrize("name", ["c4_14.cdf.gz", "gen15", "gen61", "c4_118.cdf.gz", "gen171", "c4_236.cdf.gz",
+                                  "c4_472.cdf.gz", "ieee118x8", "c5_base.cdf.gz", "ieee118x64",
+                                  "c3_base.cdfx.gz"])
+def test_cluster_lu_matches_level_launches(gb, name, precision, tol, atol):
+    grid = grid_of(gb, name)
+    out = []
+    for mode in (0, 1):
+        s = gb.Solver(grid, tolerancia=tol, no_max_iter=100, lim_inj_reat=0, metodo=0, precision=getattr(gb, precision))
+        s.set_form(gb.FORM_GRAPH)
+        s.set_lu_launch(mode)
+        out.append((s.info()["kernels_per_iteration"], s.solve(), s.solve()))
+        s.close()
+    (k0, a, a2), (k1, b, _) = out
+    assert k0 < 12 < k1
+    assert a["converged"] and b["converged"] and a["iterations"] == b["iterations"]
+    for k in ("V", "theta"):
+        np.testing.assert_allclose(a[k], b[k], rtol=0, atol=atol, err_msg=k)
+        np.testing.assert_array_equal(a[k], a2[k])  # the same bits again
+
+
+def test_cluster_lu_newton_step_and_singular(gb):
+    """gbpf_newton_step through the cluster solves J dx = g (residual against the Jacobian the library returns), and an
+    isolated bus (a zero pivot block) ends the solve with GBPF_E_SINGULAR."""
+    grid = grid_of(gb, "c4_236.cdf.gz")
+    s = gb.Solver(grid, tolerancia=1e-8, no_max_iter=100, metodo=0)
+    b = grid.buses()
+    V, th = b["V0"], b["theta0"] + 0.01 * np.sin(np.arange(grid.nB))
+    row, col, val = s.eval_jacobian(V, th)
+    n = int(row.max()) + 1
+    g = np.cos(np.arange(n))
+    dx = s.newton_step(V, th, g)
+    J = np.zeros((n, n))
+    J[row, col] = val
+    assert np.max(np.abs(J @ dx - g)) <= 1e-13 * np.abs(J).sum(1).max() * np.abs(dx).max()
+    iso = gb.create_grid(bus_type=[3, 0, 0, 0, 0], V0=[1.0] * 5, theta0=[0.0] * 5, from_bus=[1, 2, 3], to_bus=[2, 3, 4],
+                         r=[0.01] * 3, x=[0.1] * 3, Pload=[0, 0.1, 0.1, 0.1, 0.1])
+    s = gb.Solver(iso, tolerancia=1e-8, no_max_iter=10, metodo=0)
+    s.set_form(gb.FORM_GRAPH)
+    assert s.solve(full=False)["status"] == gb.E_SINGULAR
+
+
+@pytest.mark.parametrize("name", ["ieee118x4", "ieee118x16"])
+def test_persistent_form_on_request(gb, name):
+    """Grids above the persistent form's default size still run it when asked, to the graph form's answer."""
+    grid = grid_of(gb, name)
+    s = gb.Solver(grid, tolerancia=1e-8, no_max_iter=100, metodo=0)
+    assert s.form()["form"] == gb.FORM_GRAPH
+    b = grid.buses()
+    s.set_start(V0=b["V0"] * 1.001)  # before the form is built: its start is not the grid's own
+    a = s.solve()
+    s.set_form(gb.FORM_PERSISTENT)
+    assert s.form()["form"] == gb.FORM_PERSISTENT
+    p = s.solve()
+    assert a["converged"] and a["iterations"] == p["iterations"]
+    np.testing.assert_allclose(a["V"], p["V"], rtol=0, atol=1e-11)
+    np.testing.assert_allclose(a["theta"], p["theta"], rtol=0, atol=1e-11)

@@ -726,6 +726,7 @@ __global__ void k_flows(Dev d) {
 // Largest dense system of metodo = denso: a 16384 x 16384 FP64 matrix (2 GiB),
 // 8,193 buses; the right-hand side of the triangular solves sits in shared memory.
 constexpr int kDenseMaxN = 16384;
+constexpr int kDCtas = 16;  // CTAs of the dense path's clusters
 
 // ------------------------------------------------------------------ host side
 #define CK(call)                                                                     \
@@ -899,25 +900,33 @@ struct gbpf_solver {
         k_dfill<<<cdiv_int(g.nB, T), T, 0, stream>>>(d, guard);
     }
     void launch_dense_lu(int guard) {
-        const int T = 256, N = d.N;
+        const int N = d.N;
+        cudaLaunchAttribute at[1];
         for (int k0 = 0; k0 < N; k0 += kDPanel) {
-            const int k1 = std::min(N, k0 + kDPanel);
-            if (N - k0 <= kDPanelSmemRows)
-                k_dpanel_smem<<<1, kDPanelThreads,
-                                (size_t)(N - k0 + 1) * std::min(kDPanel, N - k0) * sizeof(double), stream>>>(d, k0,
-                                                                                                           guard);
-            else
+            const int nb = std::min(kDPanel, N - k0), k1 = k0 + nb, R = N - k0;
+            // rows of a CTA: an even share, no fewer than the panel's columns
+            const int rp = std::max(kDPanel, cdiv_int(R, kDCtas));
+            int ctas = 1;
+            while (ctas * rp < R) ctas *= 2;
+            if (rp <= kDPanRows) {
+                cudaLaunchConfig_t cfg = cluster_config(ctas, sizeof(double) * (size_t)rp * kDPanLd, at);
+                cfg.blockDim = dim3(kDPanClT);
+                (void)cudaLaunchKernelEx(&cfg, k_dpanel_cl, d, k0, rp, guard);
+            } else {
                 k_dpanel<<<1, kDPanelThreads, 0, stream>>>(d, k0, guard);
-            k_dlaswp<<<cdiv_int(N, T), T, 0, stream>>>(d, k0, guard);
-            if (k1 < N) {
-                k_dtrsm<<<cdiv_int(N - k1, 128), 128, 0, stream>>>(d, k0, guard);
-                const int t = cdiv_int(N - k1, 64);
-                k_dgemm<<<dim3(t, t), 256, 0, stream>>>(d, k0, guard);
             }
+            k_dswap<<<cdiv_int(N + 1 - nb, 8), 256, 0, stream>>>(d, k0, guard);
+            if (k1 < N) k_dgemm<<<dim3(cdiv_int(N + 1 - k1, 32), cdiv_int(N - k1, 64)), 256, 0, stream>>>(d, k0, guard);
         }
     }
     void launch_dense_solve(int guard) {
-        k_dsolve<<<1, kDSolveThreads, (size_t)d.N * sizeof(double), stream>>>(d, guard);
+        cudaLaunchAttribute at[1];
+        cudaLaunchConfig_t cfg = cluster_config(kDCtas, dense_back_smem(), at);
+        cfg.blockDim = dim3(kDBackThreads);
+        (void)cudaLaunchKernelEx(&cfg, k_dback, d, guard);
+    }
+    size_t dense_back_smem() const {
+        return sizeof(double) * 5 * kDPanel * (size_t)cdiv_int(cdiv_int(d.N, kDPanel), kDCtas);
     }
     void launch_eval(int guard) {  // injections, limits, mismatch
         const int T = 256;
@@ -1004,7 +1013,7 @@ gbpf_status gbpf_solver::build(const Grid &grid, const gbpf_options &o, int dev)
         d.ybus_form = g.ybus_form;
         d.N = d.dense_rule ? 2 * n : 0;
         if (d.dense_rule) {
-            d.A = A.take<double>((size_t)d.N * d.N);
+            d.A = A.take<double>((size_t)d.N * (d.N + 1));  // the right-hand side the last column
             d.ipiv = A.take<int>(d.N);
         }
         d.hist_cap = hist_cap;
@@ -1252,9 +1261,11 @@ gbpf_status gbpf_solver::ensure_graph() {
 
 gbpf_status gbpf_solver::build_graph() {
     if (d.dense_rule) {
-        CK(cudaFuncSetAttribute(k_dsolve, cudaFuncAttributeMaxDynamicSharedMemorySize, d.N * (int)sizeof(double)));
-        CK(cudaFuncSetAttribute(k_dpanel_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (kDPanelSmemRows + 1) * kDPanel * (int)sizeof(double)));
+        CK(cudaFuncSetAttribute(k_dpanel_cl, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        CK(cudaFuncSetAttribute(k_dpanel_cl, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kDPanRows * kDPanLd * (int)sizeof(double)));
+        CK(cudaFuncSetAttribute(k_dback, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        CK(cudaFuncSetAttribute(k_dback, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dense_back_smem()));
     }
     CK(cudaGraphCreate(&graph, 0));
     cudaGraphConditionalHandle h;
@@ -1301,7 +1312,7 @@ gbpf_status gbpf_solver::build_graph() {
     kernels_per_iter = (lu_fused ? 1 : nfl() + nbl() + split_levels) + 3 + 3 + (opt.lim_inj_reat && g.nPV ? 1 : 0) + 1;
     if (d.dense_rule) {
         const int panels = (d.N + kDPanel - 1) / kDPanel;
-        kernels_per_iter = 2 + 4 * panels - 2 + 2 + 3 + (opt.lim_inj_reat && g.nPV ? 1 : 0) + 1;
+        kernels_per_iter = 2 + 3 * panels - 1 + 2 + 3 + (opt.lim_inj_reat && g.nPV ? 1 : 0) + 1;
     }
     return GBPF_OK;
 }

@@ -122,3 +122,15 @@ def test_dense_rejects_grids_beyond_its_size(gb):
     with pytest.raises(gb.GbpfError) as e:
         gb.Solver(g, tolerancia=1e-8, no_max_iter=10, metodo=DENSO)
     assert e.value.status == gb.E_UNSUPPORTED
+
+
+# N = 2 (nB - 1) on both sides of a panel (32, 34, 64, 66), of the rows a CTA of the panel's cluster takes (512, 514:
+# sixteen CTAs of 32 rows, then of 33) and in between.  Both forms solve the same equations in FP64: eps kappa |dx| of
+# the last step with kappa <= 1e5 and |dx| <= 1e-2 stays below 1e-12; 1e-11.
+@pytest.mark.parametrize("nbus", [14, 17, 18, 33, 34, 101, 257, 258, 400])
+def test_dense_equals_sparse_at_panel_edges(gb, nbus):
+    grid = gb.generate(4, 5, nbus=nbus)
+    a, b = (gb.Solver(grid, tolerancia=1e-8, no_max_iter=100, metodo=m).solve() for m in (DENSO, 0))
+    assert a["converged"] and b["converged"] and a["iterations"] == b["iterations"]
+    for k in ("V", "theta"):
+        np.testing.assert_allclose(a[k], b[k], rtol=0, atol=1e-11, err_msg=k)

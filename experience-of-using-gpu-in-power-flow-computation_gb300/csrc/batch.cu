@@ -67,13 +67,31 @@ template <typename B4> __device__ __forceinline__ B4 bm(B4 a, B4 b) {
     r.z = fmx(a.z, b.x, a.w * b.z); r.w = fmx(a.z, b.y, a.w * b.w);
     return r;
 }
-template <typename B4> __device__ __forceinline__ B4 bsub(B4 a, B4 b) {
-    a.x -= b.x; a.y -= b.y; a.z -= b.z; a.w -= b.w;
-    return a;
+// c - A B and v - A w.  FP64: the product's two terms taken out of c one after
+// the other, two fused multiply-adds a component where a product and a
+// subtraction are three instructions (an FP64 instruction holds GB300's pipe
+// 16-19 cycles a warp, and the elimination levels are most of the FP64 form's).
+// FP32: the product, then the subtraction, whose rounding decides on which
+// iteration a scenario near the tolerance ends.
+__device__ __forceinline__ double4_32a bms(double4_32a c, double4_32a a, double4_32a b) {
+    c.x = fmx(-a.y, b.z, fmx(-a.x, b.x, c.x)); c.y = fmx(-a.y, b.w, fmx(-a.x, b.y, c.y));
+    c.z = fmx(-a.w, b.z, fmx(-a.z, b.x, c.z)); c.w = fmx(-a.w, b.w, fmx(-a.z, b.y, c.w));
+    return c;
 }
-template <typename B4> __device__ __forceinline__ B4 badd(B4 a, B4 b) {
-    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-    return a;
+__device__ __forceinline__ float4 bms(float4 c, float4 a, float4 b) {
+    const float4 p = bm(a, b);
+    c.x -= p.x; c.y -= p.y; c.z -= p.z; c.w -= p.w;
+    return c;
+}
+__device__ __forceinline__ double2 bmvs(double2 v, double4_32a a, double2 w) {
+    v.x = fmx(-a.y, w.y, fmx(-a.x, w.x, v.x));
+    v.y = fmx(-a.w, w.y, fmx(-a.z, w.x, v.y));
+    return v;
+}
+__device__ __forceinline__ float2 bmvs(float2 v, float4 a, float2 w) {
+    v.x -= fmx(a.x, w.x, a.y * w.y);
+    v.y -= fmx(a.z, w.x, a.w * w.y);
+    return v;
 }
 template <typename B4, typename B2> __device__ __forceinline__ B2 bmv(B4 a, B2 v) {
     B2 r;
@@ -438,9 +456,10 @@ __device__ __forceinline__ B4 diag_block(double Pk_, double Qk_, double Vk_, dou
         const double v2 = Vk_ * Vk_;
         blk.x = -Qk_ - v2 * y.y;
         if (ak) {
-            blk.y = (Pk_ + v2 * y.x) / Vk_;
+            const double iv = rcp_rn(Vk_);  // one reciprocal for two divisions
+            blk.y = (Pk_ + v2 * y.x) * iv;
             blk.z = Pk_ - v2 * y.x;
-            blk.w = (Qk_ - v2 * y.y) / Vk_;
+            blk.w = (Qk_ - v2 * y.y) * iv;
         } else {
             blk.w = 1.0;
         }
@@ -560,7 +579,10 @@ __device__ __forceinline__ typename Blk<TJ>::b4 jac_block(const TopoView &G, int
     return blk;
 }
 
-// One elimination level, shared by both Newton kernels.  NT threads take
+// One elimination level, shared by both Newton kernels.  In FP64 a warp
+// without an item skips the sums, whose instructions would hold the pipe
+// (118-bus grid, 999 instances 0.79 -> 0.74 ms a call and one solve 0.380 ->
+// 0.368 ms, with the fused products of bms).  NT threads take
 // part (t = 0..NT-1); a group of 2^lg of them shares one pivot (entry, row),
 // strides over its gather list and sums the partial updates with shuffles
 // (lane 0 of the group starts from the stored value, the others from zero, so
@@ -580,6 +602,7 @@ __device__ __forceinline__ bool lu_pivots(const TopoView &G, int l, int lg, int 
     bool sing = false;
     for (int b0 = 0; b0 < cnt; b0 += ng) {
         const int w = b0 + (t >> lg);
+        if (sizeof(TJ) == 8 && b0 + ((t & ~31) >> lg) >= cnt) break;  // none of this warp's
         const bool on = w < cnt;
         const int j = on ? G.flev_steps[beg + w] : 0;
         B4 D;
@@ -594,10 +617,8 @@ __device__ __forceinline__ bool lu_pivots(const TopoView &G, int l, int lg, int 
             for (int q = G.dg_ptr[j] + gl; q < G.dg_ptr[j + 1]; q += gs) {
                 const int p = G.dg_pos[q];
                 const B4 lj = Lv[p];
-                D = bsub(D, bm(lj, Uv[p]));
-                const B2 v = bmv(lj, ys[G.dg_k[q]]);
-                yj.x -= v.x;
-                yj.y -= v.y;
+                D = bms(D, lj, Uv[p]);
+                yj = bmvs(yj, lj, ys[G.dg_k[q]]);
             }
         for (int o = gs >> 1; o > 0; o >>= 1) {
             D = bsum_xor(D, o);
@@ -625,6 +646,7 @@ __device__ __forceinline__ void lu_entries(const TopoView &G, int l, int lg, int
     const int beg = G.fent_ptr[l], cnt = G.fent_ptr[l + 1] - beg;
     for (int b0 = 0; b0 < cnt; b0 += ng) {
         const int e = b0 + (t >> lg);
+        if (sizeof(TJ) == 8 && b0 + ((t & ~31) >> lg) >= cnt) break;  // none of this warp's
         const bool on = e < cnt;
         const int p = on ? G.fent_p[beg + e] : 0, j = on ? G.fent_j[beg + e] : 0;
         B4 aL, aU;
@@ -634,8 +656,8 @@ __device__ __forceinline__ void lu_entries(const TopoView &G, int l, int lg, int
         if (on)
             for (int r = G.og_ptr[p] + gl; r < G.og_ptr[p + 1]; r += gs) {
                 const int x = G.og_a[r], y = G.og_b[r];
-                aL = bsub(aL, bm(Lv[y], Uv[x]));
-                aU = bsub(aU, bm(Lv[x], Uv[y]));
+                aL = bms(aL, Lv[y], Uv[x]);
+                aU = bms(aU, Lv[x], Uv[y]);
             }
         for (int o = gs >> 1; o > 0; o >>= 1) {
             aL = bsum_xor(aL, o);
@@ -657,6 +679,7 @@ __device__ __forceinline__ void back_rows(const TopoView &G, int l, int lg, int 
     const int beg = G.blev_ptr[l], cnt = G.blev_ptr[l + 1] - beg;
     for (int b0 = 0; b0 < cnt; b0 += ng) {
         const int w = b0 + (t >> lg);
+        if (sizeof(TJ) == 8 && b0 + ((t & ~31) >> lg) >= cnt) break;  // none of this warp's
         const bool on = w < cnt;
         const int j = on ? G.blev_steps[beg + w] : 0;
         B2 acc;
@@ -664,9 +687,7 @@ __device__ __forceinline__ void back_rows(const TopoView &G, int l, int lg, int 
         if (on && gl == 0) acc = ys[j];
         if (on)
             for (int p = G.up_ptr[j] + gl; p < G.up_ptr[j + 1]; p += gs) {
-                const B2 v = bmv(Uv[p], ys[G.up_col[p]]);
-                acc.x -= v.x;
-                acc.y -= v.y;
+                acc = bmvs(acc, Uv[p], ys[G.up_col[p]]);
             }
         for (int o = gs >> 1; o > 0; o >>= 1) acc = b2sum_xor(acc, o);
         if (on && gl == 0) ys[j] = bmv(dinv[j], acc);
@@ -685,6 +706,7 @@ __device__ __forceinline__ void fwd_rows(const TopoView &G, int l, int lg, int t
     const int beg = G.flev_ptr[l], cnt = G.flev_ptr[l + 1] - beg;
     for (int b0 = 0; b0 < cnt; b0 += ng) {
         const int w = b0 + (t >> lg);
+        if (sizeof(TJ) == 8 && b0 + ((t & ~31) >> lg) >= cnt) break;  // none of this warp's
         const bool on = w < cnt;
         const int j = on ? G.flev_steps[beg + w] : 0;
         B2 yj;
@@ -692,9 +714,7 @@ __device__ __forceinline__ void fwd_rows(const TopoView &G, int l, int lg, int t
         if (on && gl == 0) yj = ys[j];
         if (on)
             for (int q = G.dg_ptr[j] + gl; q < G.dg_ptr[j + 1]; q += gs) {
-                const B2 v = bmv(Lv[G.dg_pos[q]], ys[G.dg_k[q]]);
-                yj.x -= v.x;
-                yj.y -= v.y;
+                yj = bmvs(yj, Lv[G.dg_pos[q]], ys[G.dg_k[q]]);
             }
         for (int o = gs >> 1; o > 0; o >>= 1) yj = b2sum_xor(yj, o);
         if (on && gl == 0) ys[j] = yj;
@@ -725,6 +745,7 @@ __device__ __forceinline__ bool lu_level1(const TopoView &G, int l, int lgp, int
         const int beg = G.flev_ptr[l], cnt = G.flev_ptr[l + 1] - beg;
         for (int b0 = 0; b0 < cnt; b0 += ng) {
             const int w = b0 + (t >> lgp);
+            if (sizeof(TJ) == 8 && b0 + ((t & ~31) >> lgp) >= cnt) break;  // none of this warp's
             const bool on = w < cnt;
             const int j = on ? G.flev_steps[beg + w] : 0;
             B4 D;
@@ -739,10 +760,8 @@ __device__ __forceinline__ bool lu_level1(const TopoView &G, int l, int lgp, int
                 for (int q = G.dg_ptr[j] + gl; q < G.dg_ptr[j + 1]; q += gs) {
                     const int p = G.dg_pos[q], k = G.dg_k[q];
                     const B4 lt = Lv[p];
-                    D = bsub(D, bm(lt, bm(dinv[k], Uv[p])));
-                    const B2 v = bmv(lt, zs[k]);
-                    yj.x -= v.x;
-                    yj.y -= v.y;
+                    D = bms(D, lt, bm(dinv[k], Uv[p]));
+                    yj = bmvs(yj, lt, zs[k]);
                 }
             for (int o = gs >> 1; o > 0; o >>= 1) {
                 D = bsum_xor(D, o);
@@ -766,6 +785,7 @@ __device__ __forceinline__ bool lu_level1(const TopoView &G, int l, int lgp, int
         const int beg = G.fent_ptr[l], cnt = G.fent_ptr[l + 1] - beg;
         for (int b0 = 0; b0 < cnt; b0 += ng) {
             const int e = b0 + (te >> lge);
+            if (sizeof(TJ) == 8 && b0 + ((te & ~31) >> lge) >= cnt) break;  // none of this warp's
             const bool on = e < cnt;
             const int p = on ? G.fent_p[beg + e] : 0;
             B4 aL, aU;
@@ -776,8 +796,8 @@ __device__ __forceinline__ bool lu_level1(const TopoView &G, int l, int lgp, int
                 for (int r = G.og_ptr[p] + gl; r < G.og_ptr[p + 1]; r += gs) {
                     const int x = G.og_a[r], y = G.og_b[r];
                     const B4 dk = dinv[G.og_k[r]];
-                    aL = bsub(aL, bm(Lv[y], bm(dk, Uv[x])));
-                    aU = bsub(aU, bm(Lv[x], bm(dk, Uv[y])));
+                    aL = bms(aL, Lv[y], bm(dk, Uv[x]));
+                    aU = bms(aU, Lv[x], bm(dk, Uv[y]));
                 }
             for (int o = gs >> 1; o > 0; o >>= 1) {
                 aL = bsum_xor(aL, o);
@@ -817,12 +837,20 @@ __device__ __forceinline__ bool lu_level1_q(const TopoView &G, int l, int lgp, i
         const double b0 = __shfl_sync(qm, b, sB0), b1 = __shfl_sync(qm, b, sB1);
         return __fma_rn(a0, b0, a1 * b1);
     };
+    // component c of acc - A B
+    auto qms = [&](double acc, double a, double b, double &a0, double &a1) {
+        a0 = __shfl_sync(qm, a, sA0);
+        a1 = __shfl_sync(qm, a, sA1);
+        const double b0 = __shfl_sync(qm, b, sB0), b1 = __shfl_sync(qm, b, sB1);
+        return __fma_rn(-a1, b1, __fma_rn(-a0, b0, acc));
+    };
     bool sing = false;
     {
         const int tl = t >> 2, gs = 1 << lgp, gl = tl & (gs - 1), ng = (NT >> 2) >> lgp;
         const int beg = G.flev_ptr[l], cnt = G.flev_ptr[l + 1] - beg;
         for (int b0 = 0; b0 < cnt; b0 += ng) {
             const int w = b0 + (tl >> lgp);
+            if (b0 + ((tl & ~7) >> lgp) >= cnt) break;  // none of this warp's
             const bool on = w < cnt;
             const int j = on ? G.flev_steps[beg + w] : 0;
             double D = 0.0, yr = 0.0;  // component c of D_j, row r of y_j
@@ -836,9 +864,9 @@ __device__ __forceinline__ bool lu_level1_q(const TopoView &G, int l, int lgp, i
                     const double lt = comp(&Lv[p]), dk = comp(&dinv[k]), u = comp(&Uv[p]);
                     double d0, d1, l0, l1;
                     const double tk = qmul(dk, u, d0, d1);  // (D_k^-1 U(k,j))_c
-                    D -= qmul(lt, tk, l0, l1);              // (Lt(j,k) D_k^-1 U(k,j))_c
+                    D = qms(D, lt, tk, l0, l1);             // - (Lt(j,k) D_k^-1 U(k,j))_c
                     const double2 z = zs[k];
-                    yr -= __fma_rn(l0, z.x, l1 * z.y);      // (Lt(j,k) z_k)_r
+                    yr = __fma_rn(-l1, z.y, __fma_rn(-l0, z.x, yr));  // - (Lt(j,k) z_k)_r
                 }
             for (int o = gs >> 1; o > 0; o >>= 1) {
                 D += __shfl_xor_sync(0xffffffffu, D, 4 * o);
@@ -868,6 +896,7 @@ __device__ __forceinline__ bool lu_level1_q(const TopoView &G, int l, int lgp, i
         const int beg = G.fent_ptr[l], cnt = G.fent_ptr[l + 1] - beg;
         for (int b0 = 0; b0 < cnt; b0 += ng) {
             const int e = b0 + (tl >> lge);
+            if (b0 + ((tl & ~7) >> lge) >= cnt) break;  // none of this warp's
             const bool on = e < cnt;
             const int p = on ? G.fent_p[beg + e] : 0;
             double aL = 0.0, aU = 0.0;
@@ -878,8 +907,8 @@ __device__ __forceinline__ bool lu_level1_q(const TopoView &G, int l, int lgp, i
                     const double dk = comp(&dinv[G.og_k[q]]);
                     const double ly = comp(&Lv[y]), ux = comp(&Uv[x]), lx = comp(&Lv[x]), uy = comp(&Uv[y]);
                     double a0, a1;
-                    aL -= qmul(ly, qmul(dk, ux, a0, a1), a0, a1);
-                    aU -= qmul(lx, qmul(dk, uy, a0, a1), a0, a1);
+                    aL = qms(aL, ly, qmul(dk, ux, a0, a1), a0, a1);
+                    aU = qms(aU, lx, qmul(dk, uy, a0, a1), a0, a1);
                 }
             for (int o = gs >> 1; o > 0; o >>= 1) {
                 aL += __shfl_xor_sync(0xffffffffu, aL, 4 * o);
@@ -911,6 +940,7 @@ __device__ __forceinline__ bool lu_pivots_q(const TopoView &G, int l, int lg, in
     bool sing = false;
     for (int b0 = 0; b0 < cnt; b0 += ng) {
         const int w = b0 + (tl >> lg);
+        if (b0 + ((tl & ~7) >> lg) >= cnt) break;  // none of this warp's
         const bool on = w < cnt;
         const int j = on ? G.flev_steps[beg + w] : 0;
         double D = 0.0, yr = 0.0;
@@ -924,9 +954,9 @@ __device__ __forceinline__ bool lu_pivots_q(const TopoView &G, int l, int lg, in
                 const double lj = comp(&Lv[p]), u = comp(&Uv[p]);
                 const double l0 = __shfl_sync(qm, lj, sA0), l1 = __shfl_sync(qm, lj, sA1);
                 const double u0 = __shfl_sync(qm, u, sB0), u1 = __shfl_sync(qm, u, sB1);
-                D -= __fma_rn(l0, u0, l1 * u1);             // (L(j,k) U(k,j))_c
+                D = __fma_rn(-l1, u1, __fma_rn(-l0, u0, D));         // - (L(j,k) U(k,j))_c
                 const double2 yk = ys[G.dg_k[q]];
-                yr -= __fma_rn(l0, yk.x, l1 * yk.y);        // (L(j,k) y_k)_r
+                yr = __fma_rn(-l1, yk.y, __fma_rn(-l0, yk.x, yr));   // - (L(j,k) y_k)_r
             }
         for (int o = gs >> 1; o > 0; o >>= 1) {
             D += __shfl_xor_sync(0xffffffffu, D, 4 * o);
@@ -957,10 +987,16 @@ __device__ __forceinline__ void lu_entries_q(const TopoView &G, int l, int lg, i
         const double b0 = __shfl_sync(qm, b, sB0), b1 = __shfl_sync(qm, b, sB1);
         return __fma_rn(a0, b0, a1 * b1);
     };
+    auto qms = [&](double acc, double a, double b) {  // component c of acc - A B
+        const double a0 = __shfl_sync(qm, a, sA0), a1 = __shfl_sync(qm, a, sA1);
+        const double b0 = __shfl_sync(qm, b, sB0), b1 = __shfl_sync(qm, b, sB1);
+        return __fma_rn(-a1, b1, __fma_rn(-a0, b0, acc));
+    };
     const int tl = t >> 2, gs = 1 << lg, gl = tl & (gs - 1), ng = (NT >> 2) >> lg;
     const int beg = G.fent_ptr[l], cnt = G.fent_ptr[l + 1] - beg;
     for (int b0 = 0; b0 < cnt; b0 += ng) {
         const int e = b0 + (tl >> lg);
+        if (b0 + ((tl & ~7) >> lg) >= cnt) break;  // none of this warp's
         const bool on = e < cnt;
         const int p = on ? G.fent_p[beg + e] : 0, j = on ? G.fent_j[beg + e] : 0;
         double aL = 0.0, aU = 0.0;
@@ -968,8 +1004,8 @@ __device__ __forceinline__ void lu_entries_q(const TopoView &G, int l, int lg, i
         if (on)
             for (int q = G.og_ptr[p] + gl; q < G.og_ptr[p + 1]; q += gs) {
                 const int x = G.og_a[q], y = G.og_b[q];
-                aL -= qmul(comp(&Lv[y]), comp(&Uv[x]));
-                aU -= qmul(comp(&Lv[x]), comp(&Uv[y]));
+                aL = qms(aL, comp(&Lv[y]), comp(&Uv[x]));
+                aU = qms(aU, comp(&Lv[x]), comp(&Uv[y]));
             }
         for (int o = gs >> 1; o > 0; o >>= 1) {
             aL += __shfl_xor_sync(0xffffffffu, aL, 4 * o);
@@ -996,6 +1032,7 @@ __device__ __forceinline__ void fwd_rows_q(const TopoView &G, int l, int lg, int
     const int beg = G.flev_ptr[l], cnt = G.flev_ptr[l + 1] - beg;
     for (int b0 = 0; b0 < cnt; b0 += ng) {
         const int w = b0 + (tl >> lg);
+        if (b0 + ((tl & ~7) >> lg) >= cnt) break;  // none of this warp's
         const bool on = w < cnt;
         const int j = on ? G.flev_steps[beg + w] : 0;
         double yr = 0.0;
@@ -1005,7 +1042,7 @@ __device__ __forceinline__ void fwd_rows_q(const TopoView &G, int l, int lg, int
                 const double lj = ((const double *)&Lv[G.dg_pos[q]])[c];
                 const double l0 = __shfl_sync(qm, lj, sA0), l1 = __shfl_sync(qm, lj, sA1);
                 const double2 yk = ys[G.dg_k[q]];
-                yr -= __fma_rn(l0, yk.x, l1 * yk.y);
+                yr = __fma_rn(-l1, yk.y, __fma_rn(-l0, yk.x, yr));
             }
         for (int o = gs >> 1; o > 0; o >>= 1) yr += __shfl_xor_sync(0xffffffffu, yr, 4 * o);
         if (on && gl == 0 && s == 0) ((double *)&ys[j])[r] = yr;

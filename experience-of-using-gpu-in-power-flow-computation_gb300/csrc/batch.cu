@@ -43,6 +43,8 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
+constexpr int kTailMaxBatch = 80;  // order of a tail (tail_lu) at most: two blocks per SM
+constexpr int kTailPanel = 4;      // its pivots to a panel
 // Iteration at which an instance still running on the warp-per-instance
 // kernel moves to a thread block of its own: a batch finishes when its slowest
 // instance does, and a warp runs one Newton iteration several times slower
@@ -128,9 +130,17 @@ struct TopoOff {
         og_ptr, og_a, og_b, flev_ptr, flev_steps, blev_ptr, blev_steps, ysl, rbus, cbus, fent_ptr, fent_p,
         fent_j, lvl_group, lvl_group_w, lvl_narrow, lvl_rot, og_k, yval32, lvl_group4, lvl_rot4, inj_order,
         lvl_group4w, lvl_q4w;
+    // the tail form of the FP32 blocks (tail_lu): levels of the steps before
+    // the tail, and what takes their updates into it
+    int t_flev_ptr, t_flev_steps, t_fent_ptr, t_fent_p, t_blev_ptr, t_blev_steps, t_group, t_rot, t_dg_end, t_sc_p, t_sc_k,
+        t_task_ptr, t_task;
 };
 struct Topo {
     int nB, nL, n, nup, nnzY, nPV, nfl, nbl, fac_smem, blob_smem, blob_bytes;
+    // tail: order of the dense trailing block that block-mode FP32 instances
+    // factor right-looking (0: none, or no room by the plan; dense: the order
+    // there is); then the forward and backward levels before it
+    int tail, dense, t_nfl, t_nbl, t_nsc;
     const char *blob;  // global copy
     const char *flat;  // the shared flat-start iteration (k_flat_start), or null
     TopoOff o;
@@ -284,7 +294,7 @@ __host__ __device__ inline size_t align_up(size_t x, size_t a) { return (x + a -
 
 // Shared-memory layout of one instance (state + optionally the factor).
 struct Layout {
-    size_t V, th, cs, sn, ef, f32, P, Q, QL, act, lim, ys, zs, fac, total;
+    size_t V, th, cs, sn, ef, f32, P, Q, QL, act, lim, ys, zs, fac, tail, total;
     size_t gtotal;  // bytes of the global state region (gs)
 };
 // with_zs: room for z = D^-1 y of the one-pass levels (lu_level1).  The
@@ -297,8 +307,10 @@ struct Layout {
 // per-bus array but the flags and y, z goes there (the phasors too, read for
 // the neighbours in the injections and the Jacobian fill), leaving shared
 // memory to the factor and the substitutions, the latency-critical part.
+// tail: order of the tail (tail_lu): its columns and a panel's inverses.
 template <typename TJ>
-__host__ __device__ inline Layout layout(int nB, int n, int nup, int nPV, int fac_smem, int with_zs, int gs = 0) {
+__host__ __device__ inline Layout layout(int nB, int n, int nup, int nPV, int fac_smem, int with_zs, int gs = 0,
+                                         int tail = 0) {
     using B4 = typename Blk<TJ>::b4;
     using B2 = typename Blk<TJ>::b2;
     constexpr bool f32_form = sizeof(TJ) == 4;
@@ -329,6 +341,7 @@ __host__ __device__ inline Layout layout(int nB, int n, int nup, int nPV, int fa
     L.zs = with_zs ? take(sizeof(B2) * n, 16) : 0;
     const size_t nq = (size_t)n + 2 * (size_t)nup;
     L.fac = fac_smem ? take(sizeof(B4) * nq, 32) : 0;
+    L.tail = tail ? take(sizeof(B4) * ((size_t)(tail + 1) * (tail | 1) + kTailPanel), 32) : 0;
     L.total = align_up(o, 32);
     return L;
 }
@@ -1086,10 +1099,235 @@ __device__ __forceinline__ bool lu_two_pass_warp(const TopoView &G, int l, bool 
     return sing;
 }
 
+// a - l w with fused products, for a sum of a few products that starts at zero
+__device__ __forceinline__ float4 bmsf(float4 a, float4 l, float4 w) {
+    a.x = fmaf(-l.x, w.x, fmaf(-l.y, w.z, a.x));
+    a.y = fmaf(-l.x, w.y, fmaf(-l.y, w.w, a.y));
+    a.z = fmaf(-l.z, w.x, fmaf(-l.w, w.z, a.z));
+    a.w = fmaf(-l.z, w.y, fmaf(-l.w, w.w, a.w));
+    return a;
+}
+__device__ __forceinline__ float4 badd(float4 a, float4 b) {
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
+// The tail of the FP32 factor on one block: steps td .. n-1 form a dense
+// trailing block of order m (every row of it full), whose levels hold one
+// pivot each -- 78 of the 90 levels of a filled 472-bus grid -- and long gather
+// lists.  The steps before it run in one-pass levels (L unscaled); their L in
+// the tail's rows is scaled, and their updates go into the tail as outer
+// products, S(i,c) -= L(i,k) U(k,c) over the rows i and columns c that step k
+// has there: eight lanes take a row i, own it for all k (no two groups meet in
+// a block of S) and read row k of the factor as one piece, where lists of pairs
+// for each block touch a line of L1 for each operand of each pair (217,000
+// cycles an iteration at 472 buses, 77,000 as pieces).  Then the tail is
+// factored right-looking in shared memory, in panels of four pivots: a block
+// of S is read and written once a panel (2,400 -> 1,600 cycles a pivot), the
+// right-hand side is column m and the rows become W = D^-1 U, so that the back
+// substitution is x = z - W x.  1,500 FP32 instances of six grids of 14 to 472
+// buses: 4.0 -> 1.8 ms.
+// The sums of a block are kept by themselves (S) and added to the block, which
+// stays in the factor, when its row or column is the next pivot's; with the
+// diagonal blocks' sums compensated the solution's error against 64 bits is
+// that of the level form (0.89 to 1.09 times, grids of 240 to 700 buses; a
+// plain running sum 1.5 to 2.2 times).  Returns true when a pivot is singular.
+__device__ __noinline__ bool tail_lu(const Topo *T, float4 *fac, int ys_at, int tail_at) {
+    extern __shared__ __align__(32) unsigned char smem_tail[];
+    float2 *ys = (float2 *)(smem_tail + ys_at);
+    float4 *S = (float4 *)(smem_tail + tail_at);
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    const int n = T->n, m = T->tail, td = n - m, ld = m | 1;
+    const char *blob = T->blob;
+    auto arr = [&](int off) { return (const int *)(blob + off); };
+    const int *up_ptr = arr(T->o.up_ptr);
+    float4 *Lv = fac + n;
+    const float4 *Uv = Lv + T->nup;
+    float4 *dt = S + (size_t)(m + 1) * ld;
+    for (int i = tid; i < (m + 1) * ld; i += kThreads) S[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    {
+        const int *p = arr(T->o.t_sc_p), *k = arr(T->o.t_sc_k);
+        for (int i = tid; i < T->t_nsc; i += kThreads) Lv[p[i]] = bm(Lv[p[i]], fac[k[i]]);
+    }
+    __syncthreads();
+    // the right-hand side and the diagonal blocks, four lanes a row: a diagonal
+    // block cancels against its sum, so what each lane's additions round off is
+    // carried along (rest)
+    for (int w0 = 0; w0 < m; w0 += kThreads / 4) {
+        const int *dp = arr(T->o.dg_ptr), *de = arr(T->o.t_dg_end), *dq = arr(T->o.dg_pos), *dk = arr(T->o.dg_k);
+        const int w = w0 + (tid >> 2);
+        float2 y = make_float2(0.f, 0.f);
+        float4 D = make_float4(0.f, 0.f, 0.f, 0.f), rest = D;
+        if (w < m)
+            for (int q = dp[td + w] + (tid & 3); q < de[w]; q += 4) {
+                const float4 l = Lv[dq[q]];
+                y = bmvs(y, l, ys[dk[q]]);
+                const float4 d = bmsf(rest, l, Uv[dq[q]]), t = badd(D, d);
+                rest = make_float4(d.x - (t.x - D.x), d.y - (t.y - D.y), d.z - (t.z - D.z), d.w - (t.w - D.w));
+                D = t;
+            }
+        for (int s = 1; s < 4; s <<= 1) {
+            y = b2sum_xor(y, s);
+            D = bsum_xor(D, s);
+            rest = bsum_xor(rest, s);
+        }
+        if (w < m && (tid & 3) == 0) {
+            S[m * ld + w] = make_float4(y.x, 0.f, y.y, 0.f);
+            S[w * ld + w] = badd(D, rest);
+        }
+    }
+    {
+        const int *tp = arr(T->o.t_task_ptr), *col = arr(T->o.up_col);
+        const int4 *tk = (const int4 *)arr(T->o.t_task);
+        const int e8 = tid & 7, g = tid >> 3, end = tp[g + 1];
+        constexpr int kAhead = 4;
+        int t0 = tp[g];
+        int4 x[kAhead / 2];
+#pragma unroll
+        for (int q = 0; q < kAhead / 2; q++) x[q] = t0 < end ? tk[t0 / 2 + q] : make_int4(0, 0, 0, 0);
+        for (; t0 < end; t0 += kAhead) {
+            float4 l[kAhead], u[kAhead];
+            int at[kAhead];
+#pragma unroll
+            for (int q = 0; q < kAhead; q++) {
+                // (no branches: the loads of all pieces go out together)
+                const int pb = q & 1 ? x[q / 2].z : x[q / 2].x, w = q & 1 ? x[q / 2].w : x[q / 2].y, cnt = w & 15;
+                const int p = pb + min(e8, max(cnt - 1, 0));
+                l[q] = Lv[pb + (w >> 4 & 255) - 128];
+                u[q] = Uv[p];
+                const int c = col[p] - td, i = w >> 12;
+                at[q] = e8 < cnt && c != i ? c * ld + i : -1;
+            }
+            const int nt = t0 + kAhead < end ? t0 / 2 + kAhead / 2 : t0 / 2;
+#pragma unroll
+            for (int q = 0; q < kAhead / 2; q++) x[q] = tk[nt + q];
+#pragma unroll
+            for (int q = 0; q < kAhead; q++) {
+                if (at[q] >= 0) S[at[q]] = bms(S[at[q]], l[q], u[q]);
+                __syncwarp(0xffu << (lane & 24));  // the next piece may hold it on another lane
+            }
+        }
+    }
+    const int pu = up_ptr[td];
+    // Panels of kTailPanel pivots.  Within one, the first half of the threads
+    // hold a column c each, the second a row i: at pivot k they bring their
+    // block of row k or column k up to date with the panel's earlier pivots,
+    // the column's W = D^-1 U and the row's L in registers; then the blocks
+    // beyond the panel take all its pivots at once.
+    constexpr int half = kThreads / 2, P = kTailPanel;
+    static_assert(kTailMaxBatch < half, "one thread for each column and each row");
+    const bool colth = tid < half;
+    bool sing = false;
+    float4 A[P];  // the thread's blocks of the panel, before any update
+    auto fetch = [&](int k0) {
+        const int e = k0 + (colth ? tid : tid - half);
+#pragma unroll
+        for (int t = 0; t < P; t++) {
+            const int k = k0 + t;
+            const int kc = min(k, m - 1), p = pu + kc * (m - 1) - kc * (kc - 1) / 2 + (min(e, m - 1) - kc - 1);
+            const float4 *src = e <= kc ? fac + td + kc : (colth ? Uv : Lv) + p;
+            A[t] = *src;  // (column m: not used)
+        }
+    };
+    fetch(0);
+    __syncthreads();
+    for (int k0 = 0; k0 < m; k0 += P) {
+        const int np = min(P, m - k0), e = k0 + (colth ? tid : tid - half);
+        const bool on = colth ? e <= m : e < m;
+        float4 mine[P];  // W(k, c) or L(i, k)
+#pragma unroll
+        for (int t = 0; t < P; t++) {
+            if (t >= np) break;
+            const int k = k0 + t;
+            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (colth) {
+                if (on && e >= k) {
+                    const float2 y = ys[td + k];
+                    const float4 a = e == m ? make_float4(y.x, 0.f, y.y, 0.f) : A[t];
+#pragma unroll
+                    for (int r = 0; r < t; r++) f = bmsf(f, S[(k0 + r) * ld + k], mine[r]);
+                    f = badd(a, badd(S[e * ld + k], f));
+                    S[e * ld + k] = f;
+                    if (e == k) {
+                        const float det = f.x * f.w - f.y * f.z;
+                        sing |= (det == 0.f || !isfinite(det));
+                        const float rd = rcp_rn(det);
+                        dt[t] = make_float4(f.w * rd, -f.y * rd, -f.z * rd, f.x * rd);
+                    }
+                }
+            } else if (on && e > k) {
+#pragma unroll
+                for (int r = 0; r < t; r++) f = bmsf(f, mine[r], bm(dt[r], S[k * ld + k0 + r]));
+                f = badd(A[t], badd(S[k * ld + e], f));
+                S[k * ld + e] = f;
+            }
+            __syncthreads();
+            mine[t] = f;
+            if (colth) mine[t] = bm(dt[t], f);
+        }
+        __syncthreads();
+        // the rows become W, for the updates below and the back substitution
+#pragma unroll
+        for (int t = 0; t < P; t++)
+            if (colth && on && t < np && e > k0 + t) S[e * ld + k0 + t] = mine[t];
+        const int nx = k0 + P;
+        if (nx >= m) break;
+        fetch(nx);
+        __syncthreads();
+        for (int c = nx + 2 * wp; c <= m; c += 2 * kWarps) {
+            const bool two = c < m;
+            float4 *s0 = S + c * ld, *s1 = two ? s0 + ld : s0;
+            float4 w0[P], w1[P];
+#pragma unroll
+            for (int t = 0; t < P; t++) {
+                w0[t] = s0[k0 + t];
+                w1[t] = s1[k0 + t];
+            }
+            for (int i = nx + lane; i < m; i += 32) {
+                float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
+#pragma unroll
+                for (int t = 0; t < P; t++) {
+                    const float4 l = S[(k0 + t) * ld + i];
+                    a0 = bmsf(a0, l, w0[t]);
+                    a1 = bmsf(a1, l, w1[t]);
+                }
+                s0[i] = badd(s0[i], a0);
+                if (two) s1[i] = badd(s1[i], a1);
+            }
+        }
+        __syncthreads();
+    }
+    __syncthreads();
+    // x = z - W x of the tail: two threads a row, x_j published and then taken
+    // out of the rows above it
+    constexpr int kBackT = (2 * kTailMaxBatch + 31) / 32 * 32;
+    static_assert(kBackT <= kThreads, "two threads a row");
+    if (tid < kBackT) {
+        const int i = tid >> 1, r = tid & 1;
+        const float z = i < m ? ((const float *)&S[m * ld + i])[2 * r] : 0.f;
+        float sum = 0.f, part = 0.f;  // of W x, and of the last eight
+        for (int j = m - 1; j >= 0; j--) {
+            if (i == j) ((float *)&ys[td + j])[r] = z - (sum + part);
+            const float *U = (const float *)&S[j * ld + min(i, m - 1)];
+            const float u0 = i < j ? U[2 * r] : 0.f, u1 = i < j ? U[2 * r + 1] : 0.f;
+            asm volatile("bar.sync 1, %0;" ::"n"(kBackT) : "memory");
+            const float2 x = ys[td + j];
+            part += fmx(u0, x.x, u1 * x.y);
+            if (!(j & 7)) {
+                sum += part;
+                part = 0.f;
+            }
+        }
+    }
+    __syncthreads();
+    return sing;
+}
+
 // GS: the state placement level of layout(); 3 = level 2 compiled for four
 // blocks per SM (64 registers a thread) instead of two.
 template <typename TJ, int GS>
 __global__ void __launch_bounds__(kThreads, GS == 3 ? 4 : 2) k_nr_block(Args a) {
+    // (at 64 registers a thread the call alone cost a 1,888-bus batch 10 %)
+    constexpr bool kTails = sizeof(TJ) == 4 && GS < 3;
     constexpr int LV = GS > 2 ? 2 : GS;
     using B4 = typename Blk<TJ>::b4;
     using B2 = typename Blk<TJ>::b2;
@@ -1127,7 +1365,7 @@ __global__ void __launch_bounds__(kThreads, GS == 3 ? 4 : 2) k_nr_block(Args a) 
         }
         const TopoView G = bind(T.o, blob);
         const long long off = a.inst_off[inst];
-        const Layout L = layout<TJ>(T.nB, T.n, T.nup, T.nPV, T.fac_smem, a.lu1, LV);
+        const Layout L = layout<TJ>(T.nB, T.n, T.nup, T.nPV, T.fac_smem, a.lu1, LV, a.lu1 ? T.tail : 0);
         // the state arrays layout() moves to global memory (LV)
         unsigned char *gst = LV ? a.gstate + (long long)blockIdx.x * a.gstate_stride : ism;
         unsigned char *vst = (LV >= 2 || (LV && sizeof(TJ) == 4)) ? gst : ism;
@@ -1314,7 +1552,38 @@ __global__ void __launch_bounds__(kThreads, GS == 3 ? 4 : 2) k_nr_block(Args a) 
                     // With lu1 each level is one pass (lu_level1: pivots and entries
                     // side by side, L unscaled) and needs one barrier instead of two.
                     B2 *zs = (B2 *)(ism + L.zs);
-                    for (int l = 0; l < T.nfl; l++) {
+                    const bool tailed = kTails && a.lu1 && T.tail && !a.narrow && !a.no_group;
+                    if constexpr (kTails) {
+                        if (tailed) {
+                            // the steps before the tail, the tail, the rows
+                            // before the tail
+                            TopoView H = G;
+                            H.flev_ptr = (const int *)(T.blob + T.o.t_flev_ptr);
+                            H.flev_steps = (const int *)(T.blob + T.o.t_flev_steps);
+                            H.fent_ptr = (const int *)(T.blob + T.o.t_fent_ptr);
+                            H.fent_p = (const int *)(T.blob + T.o.t_fent_p);
+                            H.blev_ptr = (const int *)(T.blob + T.o.t_blev_ptr);
+                            H.blev_steps = (const int *)(T.blob + T.o.t_blev_steps);
+                            const int *grp = (const int *)(T.blob + T.o.t_group);
+                            const int *rot = (const int *)(T.blob + T.o.t_rot);
+                            bool sing = false;
+                            for (int l = 0; l < T.t_nfl; l++) {
+                                sing |= lu_level1<TJ, kThreads>(H, l, grp[3 * l], grp[3 * l + 1], rot[l], tid, fac,
+                                                                dinv, ys, zs, Lv, Uv);
+                                __syncthreads();
+                            }
+                            sing |= tail_lu(&a.topo[t_id], fac, (int)((unsigned char *)ys - smem),
+                                            (int)(ism + L.tail - smem));
+                            if (sing) { s_status = GBPF_E_SINGULAR; s_done = 1; }
+                            __syncthreads();
+                            for (int l = 0; l < T.t_nbl; l++) {
+                                back_rows<TJ, kThreads>(H, l, grp[3 * l + 2], tid, dinv, Uv, ys);
+                                __syncthreads();
+                            }
+                            Ub = nullptr;  // x is there
+                        }
+                    }
+                    for (int l = 0; !tailed && l < T.nfl; l++) {
                         if (a.narrow && (G.lvl_narrow[l] & 1)) {
                             if (warp == 0) {
                                 const int gp = a.no_group ? 0 : G.lvl_group_w[3 * l];
@@ -1376,7 +1645,7 @@ __global__ void __launch_bounds__(kThreads, GS == 3 ? 4 : 2) k_nr_block(Args a) 
                 }
                 if (s_done) break;
                 // backward substitution, level by level, narrow levels on warp 0
-                for (int l = 0; l < T.nbl; l++) {
+                for (int l = 0; Ub && l < T.nbl; l++) {
                     if (a.narrow && (G.lvl_narrow[l] & 2)) {
                         if (warp == 0) {
                             back_rows<TJ, 32>(G, l, a.no_group ? 0 : G.lvl_group_w[3 * l + 2], lane, Db, Ub, ys);
@@ -2281,7 +2550,7 @@ gbpf_status gbpf_batch::add_topology(const Grid &g) {
         if (src && bytes) std::memcpy(blob.data() + o, src, bytes);
         return (int)o;
     };
-    TopoOff o;
+    TopoOff o{};
     o.yptr = put(y.rowptr.data(), (nB + 1) * 4); o.ycol = put(y.col.data(), y.nnz * 4);
     o.yval = put(nullptr, (size_t)y.nnz * 16);
     o.type = put(g.type.data(), nB * 4); o.pv_bus = put(pv0.data(), g.nPV * 4);
@@ -2406,6 +2675,113 @@ gbpf_status gbpf_batch::add_topology(const Grid &g) {
     o.lvl_rot4 = put(rot4.data(), rot4.size() * 4);
     o.lvl_group4w = put(grp4w.data(), grp4w.size() * 4);
     o.lvl_q4w = put(q4w.data(), q4w.size() * 4);
+    // the tail form (tail_lu): the dense trailing block of the factor, at most
+    // kTailMaxBatch steps; levels of the steps before it and their lanes, and
+    // which of their rows each eight threads take into it.  Behind the arrays
+    // that a block may stage: it is read where it lies.
+    const size_t blob_staged = blob.size();
+    int td = n, t_nfl = 0, t_nbl = 0, t_nsc = 0;
+    if (precision == GBPF_PREC_FP32_IR)
+        while (td > 0 && n - td < kTailMaxBatch && S.up_ptr[td] - S.up_ptr[td - 1] == n - td) td--;
+    if (n - td < gbpf::kTailMin) td = n;
+    if (td < n) {
+        std::vector<std::vector<int>> fl, bl;
+        std::vector<int> lv(n, 0);
+        auto add = [](std::vector<std::vector<int>> &v, int l, int j) {
+            if ((int)v.size() <= l) v.resize(l + 1);
+            v[l].push_back(j);
+        };
+        for (int j = 0; j < td; j++) {
+            int l = 0;
+            for (int q = S.dg_ptr[j]; q < S.dg_ptr[j + 1]; q++) l = std::max(l, lv[S.dg_k[q]] + 1);
+            add(fl, lv[j] = l, j);
+        }
+        for (int j = td - 1; j >= 0; j--) {
+            int l = 0;
+            for (int p = S.up_ptr[j]; p < S.up_ptr[j + 1]; p++)
+                if (S.up_col[p] < td) l = std::max(l, lv[S.up_col[p]] + 1);
+            add(bl, lv[j] = l, j);
+        }
+        t_nfl = (int)fl.size();
+        t_nbl = (int)bl.size();
+        std::vector<int> fp(1, 0), fs, ep(1, 0), es, bp(1, 0), bs, tg(3 * (size_t)std::max(t_nfl, t_nbl), 0), tr(t_nfl + 1, 0);
+        for (int l = 0; l < t_nfl; l++) {
+            int md = 0, mo = 0;
+            for (int j : fl[l]) {
+                fs.push_back(j);
+                md = std::max(md, S.dg_ptr[j + 1] - S.dg_ptr[j]);
+                for (int p = S.up_ptr[j]; p < S.up_ptr[j + 1]; p++) {
+                    es.push_back(p);
+                    mo = std::max(mo, (int)(S.og_ptr[p + 1] - S.og_ptr[p]));
+                }
+            }
+            fp.push_back((int)fs.size());
+            ep.push_back((int)es.size());
+            const int np = (int)fl[l].size();
+            tg[3 * l] = group_of(np, md, kThreads);
+            tg[3 * l + 1] = group_of(ep[l + 1] - ep[l], mo, kThreads);
+            const long long pb = (long long)np << tg[3 * l];
+            tr[l] = pb < kThreads ? (int)align_up((size_t)pb, 32) % kThreads : 0;
+        }
+        for (int l = 0; l < t_nbl; l++) {
+            int mu = 0;
+            for (int j : bl[l]) {
+                bs.push_back(j);
+                mu = std::max(mu, S.up_ptr[j + 1] - S.up_ptr[j]);
+            }
+            bp.push_back((int)bs.size());
+            tg[3 * l + 2] = group_of((int)bl[l].size(), mu, kThreads);
+        }
+        // each row's list cut at the tail (its steps ascend), and the entries
+        // before it that are in its rows and columns
+        std::vector<int> de(n - td), sp, sk;
+        for (int j = td; j < n; j++) {
+            int q = S.dg_ptr[j];
+            while (q < S.dg_ptr[j + 1] && S.dg_k[q] < td) q++;
+            de[j - td] = q;
+        }
+        // the pieces of eight blocks of each step's row in the tail: for each
+        // row of the tail that the step has, one task for each piece
+        struct Task { int pb, w; };
+        std::vector<std::vector<Task>> row(n - td);
+        for (int k = 0; k < td; k++) {
+            const int e = S.up_ptr[k + 1];
+            int b = S.up_ptr[k];
+            while (b < e && S.up_col[b] < td) b++;
+            for (int p = b; p < e; p++) {
+                sp.push_back(p);
+                sk.push_back(k);
+                const int i = S.up_col[p] - td;
+                for (int q = b; q < e; q += 8) row[i].push_back({q, std::min(8, e - q) | (p - q + 128) << 4 | i << 12});
+            }
+        }
+        t_nsc = (int)sp.size();
+        // rows to groups of eight threads, the longest first, and the groups of
+        // like length to one warp; lists padded to the pieces taken at a time
+        constexpr int kGroups = kThreads / 8;
+        std::vector<int> order(n - td);
+        for (int i = 0; i < n - td; i++) order[i] = i;
+        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return row[x].size() > row[y].size(); });
+        std::vector<std::vector<Task>> grp_tasks(kGroups);
+        for (int i : order) {
+            auto &v = *std::min_element(grp_tasks.begin(), grp_tasks.end(),
+                                        [](const auto &x, const auto &y) { return x.size() < y.size(); });
+            v.insert(v.end(), row[i].begin(), row[i].end());
+        }
+        std::stable_sort(grp_tasks.begin(), grp_tasks.end(), [](const auto &x, const auto &y) { return x.size() > y.size(); });
+        std::vector<int> tp(1, 0);
+        std::vector<Task> tasks;
+        for (const auto &v : grp_tasks) {
+            tasks.insert(tasks.end(), v.begin(), v.end());
+            while (tasks.size() % 4) tasks.push_back({0, 128 << 4});
+            tp.push_back((int)tasks.size());
+        }
+        auto putv = [&](const std::vector<int> &v) { return put(v.data(), v.size() * 4); };
+        o.t_flev_ptr = putv(fp); o.t_flev_steps = putv(fs); o.t_fent_ptr = putv(ep); o.t_fent_p = putv(es);
+        o.t_blev_ptr = putv(bp); o.t_blev_steps = putv(bs); o.t_group = putv(tg); o.t_rot = putv(tr);
+        o.t_dg_end = putv(de); o.t_sc_p = putv(sp); o.t_sc_k = putv(sk); o.t_task_ptr = putv(tp);
+        o.t_task = put(tasks.data(), tasks.size() * sizeof(Task));
+    }
     DevBuf mem, tmp;
     CK(cudaMalloc(&mem.p, blob.size()));
     CK(cudaMemcpyAsync(mem.p, blob.data(), blob.size(), cudaMemcpyHostToDevice, stream));
@@ -2442,7 +2818,8 @@ gbpf_status gbpf_batch::add_topology(const Grid &g) {
     CK(cudaStreamSynchronize(stream));
     Topo t{};
     t.nB = nB; t.nL = nL; t.n = n; t.nup = nup; t.nnzY = y.nnz; t.nPV = g.nPV; t.nfl = nfl; t.nbl = nbl;
-    t.blob_bytes = (int)blob.size();
+    t.blob_bytes = (int)blob_staged;
+    t.dense = n - td; t.t_nfl = t_nfl; t.t_nbl = t_nbl; t.t_nsc = t_nsc;
     t.blob = (const char *)mem.p;
     t.o = o;
     grids.push_back(g);
@@ -2634,6 +3011,12 @@ gbpf_status gbpf_batch::build_graph() {
     topo_warp = warp_ok;
     std::vector<int> wq, bq;
     for (int i = 0; i < n_inst; i++) (warp_ok[inst_topo[i]] ? wq : bq).push_back(i);
+    // the largest topologies first, so that no block or warp begins a long
+    // instance when the others have run out (1,500 instances of six grids of 14
+    // to 472 buses: 2.78 -> 2.36 ms)
+    auto larger = [&](int x, int y) { return topo_h[inst_topo[x]].nup > topo_h[inst_topo[y]].nup; };
+    std::stable_sort(bq.begin(), bq.end(), larger);
+    std::stable_sort(wq.begin(), wq.end(), larger);
     n_warp_q = (int)wq.size();
     n_block_q = (int)bq.size();
     queues.reset();
@@ -2645,34 +3028,57 @@ gbpf_status gbpf_batch::build_graph() {
     // state + factor fit in 110 KB, otherwise it lives in global scratch.
     // With plan.gstate the plan is also made with part of the state in global
     // memory (layout gs), and that one is taken when it fits more blocks per
-    // SM, or as many with more factors in shared memory.
-    const size_t budget = 110 * 1024, blob_cap = 48 * 1024;
+    // SM that have work, or as many with more factors and tails in shared
+    // memory.  A tail has its place before the factor.  With an instance per SM
+    // or fewer the factor may take the whole of shared memory (150 FP32
+    // instances of a 1,888-bus grid: 1.03 -> 0.91 ms).
+    const int per_sm = (n_block_q + dev_sm - 1) / dev_sm;  // blocks that there is work for
+    const size_t budget = per_sm <= 1 && !n_warp_q && plan.gstate == 1 ? (size_t)maxsm - 1024 : 110 * 1024;
+    const size_t blob_cap = 48 * 1024;
     size_t region = 0;
     for (size_t t = 0; t < topo_h.size(); t++) {
         Topo &T = topo_h[t];
         T.blob_smem = !warp_ok[t] && (size_t)T.blob_bytes <= blob_cap;
         if (T.blob_smem) region = std::max(region, align_up((size_t)T.blob_bytes, 32));
     }
+    // a tail is worth more than the blobs in shared memory (1,500 instances of
+    // six grids of 14 to 472 buses, all on blocks: 5.3 ms with the blobs, 1.9
+    // with the tails)
+    if (region && plan.lu1)
+        for (size_t t = 0; t < topo_h.size(); t++) {
+            const Topo &T = topo_h[t];
+            if (warp_ok[t] || !T.dense) continue;
+            const size_t least = layout<float>(T.nB, T.n, T.nup, T.nPV, 0, 1, 2, T.dense).total;
+            if (least <= budget && least + region > budget) {
+                for (auto &U : topo_h) U.blob_smem = 0;
+                region = 0;
+            }
+        }
     auto blk_fn = [&](int gs) -> const void * {
         if (fp32) return blk_kernel<float>(gs);
         return blk_kernel<double>(gs);
     };
     struct BlockPlan {
         size_t need = 0, scr = 0, gst = 0;
-        std::vector<int> fac;
-        int nfac = 0, occ = 0;
+        std::vector<int> fac, tail;
+        int nfac = 0, ntail = 0, occ = 0;
     };
     auto plan_blocks = [&](int gs, size_t budget, BlockPlan &bp) -> gbpf_status {
         bp.fac.assign(topo_h.size(), 1);
+        bp.tail.assign(topo_h.size(), 0);
         for (size_t t = 0; t < topo_h.size(); t++) {
             if (warp_ok[t]) continue;
             const Topo &T = topo_h[t];
             const int z = plan.lu1;
             const int lv = std::min(gs, 2);
-            const Layout with = fp32 ? layout<float>(T.nB, T.n, T.nup, T.nPV, 1, z, lv)
-                                     : layout<double>(T.nB, T.n, T.nup, T.nPV, 1, z, lv);
-            const Layout without = fp32 ? layout<float>(T.nB, T.n, T.nup, T.nPV, 0, z, lv)
-                                        : layout<double>(T.nB, T.n, T.nup, T.nPV, 0, z, lv);
+            auto lay = [&](int fac, int tail) {
+                return fp32 ? layout<float>(T.nB, T.n, T.nup, T.nPV, fac, z, lv, tail)
+                            : layout<double>(T.nB, T.n, T.nup, T.nPV, fac, z, lv);
+            };
+            const int tail = z && gs < 3 && region + lay(0, T.dense).total <= budget ? T.dense : 0;
+            const Layout with = lay(1, tail), without = lay(0, tail);
+            bp.tail[t] = tail;
+            bp.ntail += 10 * tail > 7 * T.nfl;
             bp.gst = std::max(bp.gst, with.gtotal);
             if (region + with.total <= budget) {
                 bp.nfac++;
@@ -2687,6 +3093,7 @@ gbpf_status gbpf_batch::build_graph() {
         if (!n_block_q || sm > (size_t)maxsm) return GBPF_OK;
         CK(cudaFuncSetAttribute(blk_fn(gs), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bp.occ, blk_fn(gs), kThreads, sm));
+        bp.occ = std::min(bp.occ, per_sm);
         return GBPF_OK;
     };
     // Placement level: gstate 2 / 3 / 4 take level 1 / 2 / 3 where it fits;
@@ -2698,6 +3105,10 @@ gbpf_status gbpf_batch::build_graph() {
     // 279 k at 5 and 217 k at 6 blocks per SM, where spills grow), and 133 k with the factor
     // given the whole of shared memory at 1 block per SM; FP64 57 k, 58 k,
     // 71 k, 71 k (3 blocks per SM).
+    // A tail that holds more than 0.7 of the levels is worth more than four
+    // blocks per SM (4,096 FP32 instances, level 3 without tails against two
+    // blocks with: 236 buses, 39 of 48 levels, 5.9 and 5.0 ms; 472 buses, 78 of
+    // 90, 26.0 and 18.7; 700 buses, 80 of 127, 69 and 81).
     BlockPlan bp;
     gbpf_status pst = plan_blocks(0, budget, bp);
     if (pst != GBPF_OK) return pst;
@@ -2707,15 +3118,18 @@ gbpf_status gbpf_batch::build_graph() {
             BlockPlan c;
             if ((pst = plan_blocks(gs, budget, c)) != GBPF_OK) return pst;
             const bool take = plan.gstate >= 2 ? (gs == plan.gstate - 1 && c.occ > 0)
-                                               : (2 * c.occ >= 3 * bp.occ && c.occ > 0) ||
-                                                     (c.occ == bp.occ && c.occ > 0 && c.nfac > bp.nfac);
+                                               : (2 * c.occ >= 3 * bp.occ && c.occ > 0 && c.ntail >= bp.ntail) ||
+                                                     (c.occ == bp.occ && c.occ > 0 && c.nfac + c.ntail > bp.nfac + bp.ntail);
             if (take) {
                 bp = c;
                 block_gs = gs;
             }
         }
     }
-    for (size_t t = 0; t < topo_h.size(); t++) topo_h[t].fac_smem = bp.fac[t];
+    for (size_t t = 0; t < topo_h.size(); t++) {
+        topo_h[t].fac_smem = bp.fac[t];
+        topo_h[t].tail = bp.tail[t];
+    }
     const size_t need = bp.need, scr = bp.scr;
     args.blob_region = (int)region;
     smem = n_block_q ? need + region : 0;
@@ -2737,6 +3151,7 @@ gbpf_status gbpf_batch::build_graph() {
         }
         const bool stage = state + region_r <= (size_t)maxsm;
         for (size_t t = 0; t < rt.size(); t++) {
+            rt[t].tail = 0;
             rt[t].fac_smem = 1;
             rt[t].blob_smem = warp_ok[t] && stage;
         }
@@ -3301,6 +3716,7 @@ extern "C" gbpf_status gbpf_batch_create(const gbpf_grid *const *grids, int n_gr
         for (auto &t : na) {
             t.blob_smem = 0;
             t.fac_smem = 0;
+            t.tail = 0;
             const Layout l = fp32 ? layout<float>(t.nB, t.n, t.nup, t.nPV, 0, 0) : layout<double>(t.nB, t.n, t.nup, t.nPV, 0, 0);
             b->na_smem.push_back(l.total);
             b->na_stride.push_back(align_up(fp32 ? scratch_bytes<float>(t.n, t.nup) : scratch_bytes<double>(t.n, t.nup),

@@ -511,3 +511,39 @@ def test_fp32_bench_scenarios_against_fp64(gb, workload, n):
     assert left_out <= (0.002 * n if workload == "c2" else 0), rec
     assert rec["max_abs_err_vs_fp64"]["V"] < 1e-7 and rec["max_abs_err_vs_fp64"]["theta"] < 1e-7, rec
     assert np.all(r32["final_mismatch"][ok] <= 1e-8)
+
+
+# The FP32 step before max|g| <= 1e-8 is below 1e-4 and its relative error eps32 kappa <= 6e-3 (kappa <= 1e5): both
+# forms end within 1e-6 of the FP64 answer, and one more step at most makes up for the rounding.
+@pytest.mark.parametrize("n", [3, 310])
+@pytest.mark.parametrize("nbus,dense", [(83, 15), (87, 16), (107, 16), (20, 19), (240, 38), (400, 67), (470, 78),
+                                        (490, 80), (600, 80)])
+def test_batch_fp32_dense_tail(gb, nbus, dense, n):
+    """FP32 thread-block instances of grids that end in a dense trailing block (tail_lu): just under and at its least
+    order, a grid that is all tail, in between, and just over and well over its largest, with shared memory for one
+    block and for two per SM, against the FP64 batch and against the level form (plan narrow)."""
+    if nbus == 20:  # every bus tied to every other
+        f, t = zip(*[(i, j) for i in range(1, 21) for j in range(i + 1, 21)])
+        grid = gb.create_grid(bus_type=[3] + [0] * 19, V0=[1.0] * 20, theta0=[0.0] * 20, from_bus=f, to_bus=t,
+                              r=[0.02] * 190, x=[0.2 + 0.001 * k for k in range(190)],
+                              Pload=[0.0] + [0.1 + 0.02 * k for k in range(19)], Qload=[0.0] + [0.05] * 19)
+    else:
+        grid = gb.generate(4, 11, nbus=nbus)
+    base = grid.buses()
+    lf = np.random.default_rng(nbus).uniform(0.9, 1.1, (n, grid.nB))
+    Pl, Ql, Pg = base["Pload"] * lf, base["Qload"] * lf, np.tile(base["Pg"], (n, 1))
+    out = []
+    for prec, plan in ((gb.PREC_FP64, dict(warp_mode=0)), (gb.PREC_FP32_IR, dict(warp_mode=0)),
+                       (gb.PREC_FP32_IR, dict(warp_mode=0, narrow=1))):
+        b = gb.Batch([grid], precision=prec, tolerancia=1e-8, no_max_iter=30, lim_inj_reat=0)
+        b.set_plan(**plan)
+        b.set_instances(np.zeros(n, np.int32), Pload=Pl.ravel(), Qload=Ql.ravel(), Pg=Pg.ravel())
+        b.solve()
+        out.append(b.results())
+        b.solve()
+        np.testing.assert_array_equal(b.results()["V"], out[-1]["V"])  # the same bits again
+    ref = out[0]
+    for r in out[1:]:
+        assert (r["status"] == 0).all() and (r["iterations"] <= ref["iterations"] + 1).all()
+        for k in ("V", "theta"):
+            np.testing.assert_allclose(r[k], ref[k], rtol=0, atol=1e-6, err_msg=k)

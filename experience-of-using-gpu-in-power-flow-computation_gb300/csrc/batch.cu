@@ -297,7 +297,9 @@ struct Layout {
     size_t V, th, cs, sn, ef, f32, P, Q, QL, act, lim, ys, zs, fac, tail, total;
     size_t gtotal;  // bytes of the global state region (gs)
 };
-// with_zs: room for z = D^-1 y of the one-pass levels (lu_level1).  The
+// with_zs: room for z = D^-1 y of the one-pass levels (lu_level1; FP32 takes
+// z from D^-1 and y again, the same bits, which leaves 15 KB of a 1,888-bus
+// block to L1: 6.98 -> 6.78 ms for 2,048 instances).  The
 // inverse of diagonal block j overwrites fac[j] once the block is factored.
 // gs = 1: the per-bus arrays that no thread reads for another bus's row --
 // theta, P, Q, QL and, in the FP32-LU form (whose Jacobian reads the FP32
@@ -338,7 +340,7 @@ __host__ __device__ inline Layout layout(int nB, int n, int nup, int nPV, int fa
     // ys: the mismatch, then (forward) the substituted right-hand side, then
     // (backward, in place) the Newton step
     L.ys = take(sizeof(B2) * n, 16);
-    L.zs = with_zs ? take(sizeof(B2) * n, 16) : 0;
+    L.zs = with_zs && sizeof(TJ) == 8 ? take(sizeof(B2) * n, 16) : 0;
     const size_t nq = (size_t)n + 2 * (size_t)nup;
     L.fac = fac_smem ? take(sizeof(B4) * nq, 32) : 0;
     L.tail = tail ? take(sizeof(B4) * ((size_t)(tail + 1) * (tail | 1) + kTailPanel), 32) : 0;
@@ -772,9 +774,12 @@ __device__ __forceinline__ bool lu_level1(const TopoView &G, int l, int lgp, int
             if (on)
                 for (int q = G.dg_ptr[j] + gl; q < G.dg_ptr[j + 1]; q += gs) {
                     const int p = G.dg_pos[q], k = G.dg_k[q];
-                    const B4 lt = Lv[p];
-                    D = bms(D, lt, bm(dinv[k], Uv[p]));
-                    yj = bmvs(yj, lt, zs[k]);
+                    const B4 lt = Lv[p], dk = dinv[k];
+                    B2 z;
+                    if constexpr (sizeof(TJ) == 8) z = zs[k];
+                    else z = bmv(dk, ys[k]);
+                    D = bms(D, lt, bm(dk, Uv[p]));
+                    yj = bmvs(yj, lt, z);
                 }
             for (int o = gs >> 1; o > 0; o >>= 1) {
                 D = bsum_xor(D, o);
@@ -788,7 +793,7 @@ __device__ __forceinline__ bool lu_level1(const TopoView &G, int l, int lgp, int
                 inv.x = D.w * rd; inv.y = -D.y * rd; inv.z = -D.z * rd; inv.w = D.x * rd;
                 dinv[j] = inv;
                 ys[j] = yj;
-                zs[j] = bmv(inv, yj);
+                if constexpr (sizeof(TJ) == 8) zs[j] = bmv(inv, yj);
             }
         }
     }
@@ -2492,6 +2497,7 @@ struct gbpf_batch {
     } plan;
     int block_gs = 0;  // placement level of the block-mode launch's state (layout gs)
     int warp_gs = 0;   // ... and of the warp launch's
+    int block_carve = -1, warp_carve = -1;  // division of L1 and shared memory that they ask for
     DevBuf gstate_mem, warp_gstate_mem;
     gbpf_status rebuild() {
         CK(cudaStreamSynchronize(stream));
@@ -2914,6 +2920,23 @@ gbpf_status gbpf_batch::set_instances(int n, const int *tofi, const double *Ploa
 
 gbpf_status gbpf_batch::launch(cudaStream_t st) { return launch_with(st, args, wargs, true); }
 
+// carve: share of the SM's L1 and shared memory, in percent, that the launch
+// asks for as shared memory (-1: the driver's choice)
+static void launch_kernel(const void *fn, int grid, int threads, size_t smem, cudaStream_t st, const Args &a, int carve) {
+    cudaLaunchConfig_t c{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at.val.sharedMemCarveout = (unsigned)carve;
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = carve >= 0;
+    void *args[] = {(void *)&a};
+    cudaLaunchKernelExC(&c, fn, args);
+}
+
 // One persistent launch per mode over the queues of ba (blocks) and wa (warps).
 gbpf_status gbpf_batch::launch_with(cudaStream_t st, const Args &ba, const Args &wa, bool timed) {
     const bool fp32 = precision == GBPF_PREC_FP32_IR;
@@ -2922,17 +2945,8 @@ gbpf_status gbpf_batch::launch_with(cudaStream_t st, const Args &ba, const Args 
         CK(cudaEventRecord(fork, st));
         CK(cudaStreamWaitEvent(side, fork, 0));
         if (timed) CK(cudaEventRecordWithFlags(kev[0], side, cudaEventRecordExternal));
-        if (fp32) {
-            if (block_gs == 3) k_nr_block<float, 3><<<grid_blocks, kThreads, smem, side>>>(ba);
-            else if (block_gs == 2) k_nr_block<float, 2><<<grid_blocks, kThreads, smem, side>>>(ba);
-            else if (block_gs == 1) k_nr_block<float, 1><<<grid_blocks, kThreads, smem, side>>>(ba);
-            else k_nr_block<float, 0><<<grid_blocks, kThreads, smem, side>>>(ba);
-        } else {
-            if (block_gs == 3) k_nr_block<double, 3><<<grid_blocks, kThreads, smem, side>>>(ba);
-            else if (block_gs == 2) k_nr_block<double, 2><<<grid_blocks, kThreads, smem, side>>>(ba);
-            else if (block_gs == 1) k_nr_block<double, 1><<<grid_blocks, kThreads, smem, side>>>(ba);
-            else k_nr_block<double, 0><<<grid_blocks, kThreads, smem, side>>>(ba);
-        }
+        launch_kernel(fp32 ? blk_kernel<float>(block_gs) : blk_kernel<double>(block_gs), grid_blocks, kThreads, smem, side,
+                      ba, block_carve);
         {
             const cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) {
@@ -2950,18 +2964,8 @@ gbpf_status gbpf_batch::launch_with(cudaStream_t st, const Args &ba, const Args 
     }
     if (wa.queue_len) {
         if (timed) CK(cudaEventRecordWithFlags(kev[2], st, cudaEventRecordExternal));
-        const dim3 wg(warp_grid), wb(32 * warp_warps);
-        if (fp32) {
-            if (warp_gs == 3) k_nr_warp<float, 3><<<wg, wb, warp_smem, st>>>(wa);
-            else if (warp_gs == 2) k_nr_warp<float, 2><<<wg, wb, warp_smem, st>>>(wa);
-            else if (warp_gs == 1) k_nr_warp<float, 1><<<wg, wb, warp_smem, st>>>(wa);
-            else k_nr_warp<float, 0><<<wg, wb, warp_smem, st>>>(wa);
-        } else {
-            if (warp_gs == 3) k_nr_warp<double, 3><<<wg, wb, warp_smem, st>>>(wa);
-            else if (warp_gs == 2) k_nr_warp<double, 2><<<wg, wb, warp_smem, st>>>(wa);
-            else if (warp_gs == 1) k_nr_warp<double, 1><<<wg, wb, warp_smem, st>>>(wa);
-            else k_nr_warp<double, 0><<<wg, wb, warp_smem, st>>>(wa);
-        }
+        launch_kernel(fp32 ? warp_kernel<float>(warp_gs) : warp_kernel<double>(warp_gs), warp_grid, 32 * warp_warps,
+                      warp_smem, st, wa, warp_carve);
         CK_LAUNCH();
         if (timed) CK(cudaEventRecordWithFlags(kev[3], st, cudaEventRecordExternal));
         if (wa.handoff_it > 0) {
@@ -3023,6 +3027,20 @@ gbpf_status gbpf_batch::build_graph() {
     CK(cudaMalloc(&queues.p, 4 * (size_t)n_inst + 256));
     if (n_warp_q) CK(cudaMemcpy(queues.p, wq.data(), 4 * wq.size(), cudaMemcpyHostToDevice));
     if (n_block_q) CK(cudaMemcpy((int *)queues.p + n_warp_q, bq.data(), 4 * bq.size(), cudaMemcpyHostToDevice));
+    // Where one kernel has the SMs to itself, it asks for the shared memory of
+    // its blocks and no more: the rest is L1, where the index lists and global
+    // factors are read from; left alone, the driver makes room for as many
+    // blocks as would fit (2,048 FP32 instances of a 1,888-bus grid 6.78 ->
+    // 6.60 ms, 57 buses at one warp to a block 0.20 -> 0.165).  When both run,
+    // the choice stays the driver's: an SM takes a block only when its division
+    // suits.
+    int sm_smem = 0;
+    CK(cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
+    auto carve_of = [&](int blocks, size_t dyn) {  // blocks of dyn bytes and static and reserved ones
+        const size_t want = 100 * (size_t)blocks * (dyn + 1280);
+        return (int)std::min<size_t>(100, (want + sm_smem - 1) / sm_smem);
+    };
+    block_carve = warp_carve = -1;
     // Block-mode shared-memory plan: the blob is staged in shared memory when
     // at most 48 KB; the factor stays in shared memory when blob region +
     // state + factor fit in 110 KB, otherwise it lives in global scratch.
@@ -3181,6 +3199,7 @@ gbpf_status gbpf_batch::build_graph() {
     gstate_mem.reset();
     args.gstate = nullptr;
     args.gstate_stride = block_gs ? (long long)align_up(bp.gst, 256) : 0;
+    if (n_block_q && !n_warp_q) block_carve = carve_of((grid_blocks + dev_sm - 1) / dev_sm, smem);
     if (block_gs) {
         CK(cudaMalloc(&gstate_mem.p, (size_t)args.gstate_stride * grid_blocks));
         args.gstate = (unsigned char *)gstate_mem.p;
@@ -3191,12 +3210,19 @@ gbpf_status gbpf_batch::build_graph() {
     // 1 = a level with at least 1.5x the warps per SM.  Measured on 32,768
     // instances of a 118-bus grid: FP32 level 0 8 warps per SM, warp kernel
     // 8.14 ms; level 2 16 warps per SM, 6.65 ms; FP64 level 0 7 warps per SM
-    // 25.3 ms, level 2 8 warps per SM 25.8 ms.
+    // 25.3 ms, level 2 8 warps per SM 25.8 ms.  A batch that does not fill the
+    // SMs spreads over all of them, as few warps to a block as that takes, with
+    // its state in shared memory: a warp is a serial chain, and eight on one SM
+    // share its FP64 pipes while other SMs idle (300 instances on eight warps a
+    // block and on two: 14 buses FP32 0.077 -> 0.064 ms, 57 buses 0.276 ->
+    // 0.166, 118 buses 0.327 -> 0.203, FP64 0.526 -> 0.384; the lines meet at
+    // eight warps per SM, 1,216 instances).
     warp_grid = 0;
     warp_gs = 0;
     size_t warp_gstride = 0;
     if (n_warp_q) {
         struct WarpPlan { int warps = 0, occ = 0; size_t slice = 0, gst = 0; };
+        const int per_sm_w = (n_warp_q + dev_sm - 1) / dev_sm;
         auto plan_warps = [&](int gs, WarpPlan &wp) -> gbpf_status {
             const int lv = std::min(gs, 2);
             for (size_t t = 0; t < topo_h.size(); t++) {
@@ -3209,6 +3235,7 @@ gbpf_status gbpf_batch::build_graph() {
             }
             wp.warps = (int)std::max<size_t>(1, std::min<size_t>(kWarpsMax, (size_t)maxsm / wp.slice));
             if (plan.warp_warps > 0) wp.warps = std::min(wp.warps, plan.warp_warps);
+            wp.warps = std::min(wp.warps, per_sm_w);
             const size_t sm = (size_t)wp.warps * wp.slice;
             const void *fn = fp32 ? warp_kernel<float>(gs) : warp_kernel<double>(gs);
             CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -3223,7 +3250,8 @@ gbpf_status gbpf_batch::build_graph() {
                 WarpPlan c;
                 if ((wst = plan_warps(gs, c)) != GBPF_OK) return wst;
                 const bool take = plan.warp_gstate >= 2 ? (gs == plan.warp_gstate - 1 && c.occ > 0)
-                                                        : 2 * c.occ * c.warps >= 3 * wp.occ * wp.warps;
+                                                        : wp.occ * wp.warps < per_sm_w &&
+                                                              2 * c.occ * c.warps >= 3 * wp.occ * wp.warps;
                 if (take) {
                     wp = c;
                     warp_gs = gs;
@@ -3234,6 +3262,7 @@ gbpf_status gbpf_batch::build_graph() {
         warp_warps = wp.warps;
         warp_smem = (size_t)warp_warps * slice;
         warp_grid = std::max(1, std::min((n_warp_q + warp_warps - 1) / warp_warps, dev_sm * std::max(wp.occ, 1)));
+        if (!n_block_q) warp_carve = carve_of((warp_grid + dev_sm - 1) / dev_sm, warp_smem);
         warp_gstride = warp_gs ? align_up(wp.gst, 256) : 0;
     }
     warp_gstate_mem.reset();

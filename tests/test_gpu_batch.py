@@ -547,3 +547,27 @@ def test_batch_fp32_dense_tail(gb, nbus, dense, n):
         assert (r["status"] == 0).all() and (r["iterations"] <= ref["iterations"] + 1).all()
         for k in ("V", "theta"):
             np.testing.assert_allclose(r[k], ref[k], rtol=0, atol=1e-6, err_msg=k)
+
+
+@pytest.mark.parametrize("prec", ["PREC_FP64", "PREC_FP32_IR"])
+def test_batch_spread_over_the_sms_is_exact(gb, prec):
+    """However many warps to a block a batch gets (as few as spread it over the SMs: one up to an instance per SM,
+    eight, the plan's most, from there times eight on), an instance's answer has the same bits."""
+    grid = gb.generate(4, 5, nbus=30)
+    base = grid.buses()
+    sms = int(gb.device_info()["props"][5])
+    counts = [1, sms, sms + 1, 7 * sms + 1, 8 * sms + 1]
+    lf = np.random.default_rng(2).uniform(0.8, 1.2, (counts[-1], grid.nB))
+    Pl, Ql, Pg = base["Pload"] * lf, base["Qload"] * lf, np.tile(base["Pg"], (len(lf), 1))
+    ref, used = None, []
+    for n in counts[::-1]:
+        b = gb.Batch([grid], precision=getattr(gb, prec), tolerancia=1e-8, no_max_iter=30, lim_inj_reat=0)
+        b.set_instances(np.zeros(n, np.int32), Pload=Pl[:n].ravel(), Qload=Ql[:n].ravel(), Pg=Pg[:n].ravel())
+        b.solve()
+        used.append(b.plan()["warps_per_block_used"])
+        r = b.results()
+        ref = ref or r
+        for k in ("iterations", "status", "V", "theta"):
+            got = r[k].reshape(n, -1)
+            np.testing.assert_array_equal(got, np.asarray(ref[k]).reshape(counts[-1], -1)[:n], err_msg=k)
+    assert used[::-1] == [1, 1, 2, 8, 8]

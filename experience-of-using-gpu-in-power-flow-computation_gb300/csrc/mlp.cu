@@ -18,9 +18,10 @@
 //     TMEM lanes 32w..32w+31 = output rows) and run a fused epilogue.
 // Backward products need A^T or B^T; the epilogues that produce an operand
 // also write its transpose (coalesced: 32 lanes = 32 consecutive rows).  The
-// weight-gradient GEMMs store fp32 gradients; one streaming kernel (k_adam)
-// then updates every weight, and k_transpose_bf16 refreshes the transposed
-// bf16 copies of the hidden layers' weights.
+// weight-gradient GEMMs store fp32 gradients; a streaming kernel (k_adam)
+// then updates the weights, and k_transpose_bf16 refreshes the transposed
+// bf16 copies that the input gradients read.  The training graph runs what
+// does not wait for one another side by side (gbpf_mlp::backward).
 //
 // Every wait on an mbarrier is bounded.  The operand ring's waits take the
 // launch's limit (EpiArgs::wait, set per network by gbpf_mlp_set_wait_limit;
@@ -487,8 +488,8 @@ struct BiasJobs {
 
 // Bias gradient = column sum of dZ over the batch = row sum of dZ^T; then
 // Adam on the bias (or store the gradient).  One warp per bias entry.
-__global__ void k_bias(BiasJobs J, const int *adam_t, const float *sched, float lr, float b1, float b2, float eps,
-                       int adam) {
+__global__ void k_bias(BiasJobs J, const int *adam_t, int step, const float *sched, float lr, float b1, float b2,
+                       float eps, int adam) {
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (gw >= J.row_start[J.njobs]) return;
     int j = 0;
@@ -500,7 +501,7 @@ __global__ void k_bias(BiasJobs J, const int *adam_t, const float *sched, float 
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane) return;
     if (!adam) { J.gout[j][r] = s; return; }
-    const int ti = *adam_t + 1;
+    const int ti = *adam_t + 1 + step;
     const float t = (float)ti;
     const float m = b1 * J.bm[j][r] + (1.f - b1) * s, v = b2 * J.bv[j][r] + (1.f - b2) * s * s;
     J.bm[j][r] = m;
@@ -508,13 +509,15 @@ __global__ void k_bias(BiasJobs J, const int *adam_t, const float *sched, float 
     J.b[j][r] -= sched_lr(lr, sched, ti) * (m / (1.f - powf(b1, t))) / (sqrtf(v / (1.f - powf(b2, t))) + eps);
 }
 
-// Adam on every layer's weights in one streaming pass, after the
+// Adam on the weights of several layers in one streaming pass, after the
 // weight-gradient GEMMs stored their fp32 gradients: each weight's gradient,
 // master copy and two moments are read once and the master, moments and bf16
 // copy written once, four weights a thread and kAdamU groups of them in
-// flight (evict-first: 0.8 GB a step for the 1,888-bus network, more than the
-// L2).  In the GEMM's epilogue the same update ran tile by tile between main
-// loops and reached a third of the HBM bandwidth.
+// flight (evict-first: 0.6 GB a step for the 1,888-bus network, more than the
+// L2; 86 us, 6.5 TB/s).  In the GEMM's epilogue the same update ran tile by
+// tile between main loops and reached a third of the HBM bandwidth.  `step`:
+// steps since *adam_t was advanced (once a graph launch: the update of one
+// step runs into the next).
 constexpr int kMaxAdamJobs = 9;  // up to 7 hidden layers + the output layer + the skip
 struct AdamJobs {
     const float *g[kMaxAdamJobs];
@@ -525,9 +528,9 @@ struct AdamJobs {
 };
 constexpr int kAdamU = 4;
 
-__global__ void __launch_bounds__(256) k_adam(AdamJobs J, const int *adam_t, const float *sched, float lr, float b1,
-                                              float b2, float eps) {
-    const int ti = *adam_t + 1;
+__global__ void __launch_bounds__(256) k_adam(AdamJobs J, const int *adam_t, int step, const float *sched, float lr,
+                                              float b1, float b2, float eps) {
+    const int ti = *adam_t + 1 + step;
     const float t = (float)ti, lrt = sched_lr(lr, sched, ti);
     const float c1 = 1.f / (1.f - powf(b1, t)), c2 = 1.f / (1.f - powf(b2, t));
     const long long total = J.start[J.njobs], stride = (long long)gridDim.x * blockDim.x;
@@ -571,7 +574,7 @@ __global__ void __launch_bounds__(256) k_adam(AdamJobs J, const int *adam_t, con
     }
 }
 
-__global__ void k_step(int *t) { *t += 1; }
+__global__ void k_step(int *t, int steps) { *t += steps; }
 
 // rows of X (bf16, row length a multiple of 8) in the order perm[]
 __global__ void k_gather_bf16(const bf16 *X, int ld, const int *perm, int n, bf16 *out) {
@@ -606,8 +609,17 @@ __global__ void k_transpose_batches(const bf16 *Xs, int kin, int B, bf16 *XT) {
     }
 }
 // Wt [cols, rows] = W^T for bf16 W [rows, cols], through 32 x 32 tiles.
-__global__ void k_transpose_bf16(const bf16 *W, int rows, int cols, bf16 *Wt) {
+struct TransposeJobs {
+    const bf16 *W[kMaxAdamJobs];
+    bf16 *Wt[kMaxAdamJobs];
+    int rows[kMaxAdamJobs], cols[kMaxAdamJobs];
+};
+// (blockIdx.z: the matrix; the grid covers the largest)
+__global__ void k_transpose_bf16(TransposeJobs J) {
     __shared__ bf16 tile[32][34];
+    const bf16 *W = J.W[blockIdx.z];
+    bf16 *Wt = J.Wt[blockIdx.z];
+    const int rows = J.rows[blockIdx.z], cols = J.cols[blockIdx.z];
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
     for (int y = threadIdx.y; y < 32; y += blockDim.y) {
         const int r = r0 + y, c = c0 + threadIdx.x;
@@ -772,8 +784,8 @@ struct gbpf_mlp {
     // split-K workspace of the training GEMMs: one 128 x 128 fp32 partial per
     // CTA (at most one CTA per SM splits) and one arrival counter per tile
     Dev splitk;
-    float *ws = nullptr;
-    int *ws_cnt = nullptr;
+    float *ws[3] = {};    // ... for the chain, the side and the hidden weight gradients (Fork)
+    int *ws_cnt[3] = {};
     std::vector<float> in_mean, in_iscale, out_mean, out_scale;  // host copies
     float *d_in_mean = nullptr, *d_in_iscale = nullptr, *d_out_mean = nullptr, *d_out_scale = nullptr;
     int *d_t = nullptr, *d_err = nullptr;
@@ -791,6 +803,14 @@ struct gbpf_mlp {
     Work tw;
     int graph_B = 0, graph_steps = 0;
     cudaGraphExec_t exec = nullptr;
+    // the streams that the training graph is captured on, next to each other
+    // (Fork), with a split-K workspace each
+    struct Fork {
+        cudaStream_t chain = nullptr, side = nullptr, wgrad = nullptr;
+        cudaEvent_t begin = nullptr, out = nullptr, used = nullptr, chained = nullptr, updated = nullptr, hidden = nullptr;
+        std::vector<cudaEvent_t> dz;
+        int side_open = 0;  // an update on `side` that the chain has not waited for
+    } fk;
     // inference workspace
     Work iw;
     int iw_cap = 0;
@@ -807,6 +827,12 @@ struct gbpf_mlp {
 
     ~gbpf_mlp() {
         if (exec) cudaGraphExecDestroy(exec);
+        for (cudaStream_t q : {fk.chain, fk.side, fk.wgrad})
+            if (q) cudaStreamDestroy(q);
+        for (cudaEvent_t q : {fk.begin, fk.out, fk.used, fk.chained, fk.updated, fk.hidden})
+            if (q) cudaEventDestroy(q);
+        for (cudaEvent_t q : fk.dz)
+            if (q) cudaEventDestroy(q);
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
         if (stream) cudaStreamDestroy(stream);
@@ -816,8 +842,12 @@ struct gbpf_mlp {
     int n_layers() const { return n_hidden + 1; }  // layers of the network proper (without the skip)
     gbpf_status make_work(Work &w, int B, bool train);
     gbpf_status forward(cudaStream_t st, Work &w, const CUtensorMap &mX, int x_row0, int M, const float *target,
-                        int t_row0, float *out, bool train);
-    gbpf_status backward(cudaStream_t st, Work &w, const CUtensorMap &mXT, int xt_row0, int M, bool adam);
+                        int t_row0, float *out, bool train, Fork *f = nullptr);
+    gbpf_status backward(cudaStream_t st, Work &w, const CUtensorMap &mXT, int xt_row0, int M, bool adam, int step = 0,
+                         Fork *f = nullptr);
+    gbpf_status make_fork();
+    gbpf_status adam_layers(cudaStream_t st, std::initializer_list<std::pair<int, int>> layers, int step);
+    gbpf_status transpose_layers(cudaStream_t st, int from, int to);
     gbpf_status upload_norm();
 };
 
@@ -890,11 +920,14 @@ gbpf_status gbpf_mlp::init(int n_in_, int hidden_, int n_hidden_, int n_out_, in
     {
         int sms = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-        const size_t part = (size_t)BM * BN * sizeof(float);
-        CK(cudaMalloc(&splitk.p, (size_t)sms * part + 4 * (size_t)sms));
-        ws = (float *)splitk.p;
-        ws_cnt = (int *)((char *)splitk.p + (size_t)sms * part);
-        CK(cudaMemset(ws_cnt, 0, 4 * (size_t)sms));
+        const size_t part = (size_t)BM * BN * sizeof(float) * sms;
+        CK(cudaMalloc(&splitk.p, 3 * (part + 4 * (size_t)sms)));
+        int *cnt = (int *)((char *)splitk.p + 3 * part);
+        CK(cudaMemset(cnt, 0, 3 * 4 * (size_t)sms));
+        for (int q = 0; q < 3; q++) {
+            ws[q] = (float *)((char *)splitk.p + q * part);
+            ws_cnt[q] = cnt + q * sms;
+        }
     }
     d_t = (int *)misc.p;
     d_err = d_t + 1;
@@ -961,13 +994,13 @@ gbpf_status gbpf_mlp::make_work(Work &w, int B, bool train) {
 // target rows t_row0.. and accumulates the squared error.  Inference: the
 // output layer writes out [M, outp].
 gbpf_status gbpf_mlp::forward(cudaStream_t st, Work &w, const CUtensorMap &mX, int x_row0, int M, const float *target,
-                              int t_row0, float *out, bool train) {
+                              int t_row0, float *out, bool train, Fork *f) {
     const int nl = n_hidden + 1;
     for (int l = 0; l < nl; l++) {
         EpiArgs e{};
         e.err = d_err;
         e.wait = wait_cycles;
-        if (train) { e.ws = ws; e.ws_cnt = ws_cnt; }
+        if (train) { e.ws = ws[0]; e.ws_cnt = ws_cnt[0]; }
         e.bias = L[l].b;
         e.a_row0 = l == 0 ? x_row0 : 0;
         const CUtensorMap &ta = l == 0 ? mX : w.mH[l - 1];
@@ -995,6 +1028,8 @@ gbpf_status gbpf_mlp::forward(cudaStream_t st, Work &w, const CUtensorMap &mX, i
             e.out = out; e.ldo = outp;
         }
         gbpf_status s;
+        // the last step's update of this layer's weights
+        if (f && l == nl - 1 && f->side_open) CK(cudaStreamWaitEvent(st, f->updated, 0));
         if (l == nl - 1 && has_skip) {
             e.a2_row0 = x_row0;
             s = gemm2(st, ta, L[l].mW, mX, L[nl].mW, M, L[l].out, L[l].in, kin, e);
@@ -1008,8 +1043,8 @@ gbpf_status gbpf_mlp::forward(cudaStream_t st, Work &w, const CUtensorMap &mX, i
         EpiArgs e{};
         e.err = d_err;
         e.wait = wait_cycles;
-        e.ws = ws;
-        e.ws_cnt = ws_cnt;
+        e.ws = ws[0];
+        e.ws_cnt = ws_cnt[0];
         e.mode = EPI_PROJ;
         e.loss = d_loss;
         e.H = w.Rb; e.ldh = w.kp;
@@ -1018,8 +1053,8 @@ gbpf_status gbpf_mlp::forward(cudaStream_t st, Work &w, const CUtensorMap &mX, i
         EpiArgs g{};
         g.err = d_err;
         g.wait = wait_cycles;
-        g.ws = ws;
-        g.ws_cnt = ws_cnt;
+        g.ws = ws[0];
+        g.ws_cnt = ws_cnt[0];
         g.mode = EPI_LOSS_GRAD;
         g.lam = lam;
         g.gscale = 2.f / ((float)M * (float)n_out);
@@ -1030,78 +1065,114 @@ gbpf_status gbpf_mlp::forward(cudaStream_t st, Work &w, const CUtensorMap &mX, i
     return GBPF_OK;
 }
 
+gbpf_status gbpf_mlp::make_fork() {
+    if (fk.chain) return GBPF_OK;
+    int lo = 0, hi = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    CK(cudaStreamCreateWithPriority(&fk.side, cudaStreamNonBlocking, lo));
+    CK(cudaStreamCreateWithPriority(&fk.wgrad, cudaStreamNonBlocking, std::max(hi, lo - 1)));
+    for (cudaEvent_t *q : {&fk.begin, &fk.out, &fk.used, &fk.chained, &fk.updated, &fk.hidden})
+        CK(cudaEventCreateWithFlags(q, cudaEventDisableTiming));
+    fk.dz.assign(n_hidden, nullptr);
+    for (auto &q : fk.dz) CK(cudaEventCreateWithFlags(&q, cudaEventDisableTiming));
+    CK(cudaStreamCreateWithPriority(&fk.chain, cudaStreamNonBlocking, hi));
+    return GBPF_OK;
+}
+
+// Adam on the weights of layers [first, second) of each range.  Blocks take
+// one piece each and go: a grid that loops keeps the SMs from the GEMMs that
+// run next to it.
+gbpf_status gbpf_mlp::adam_layers(cudaStream_t st, std::initializer_list<std::pair<int, int>> layers, int step) {
+    AdamJobs A{};
+    A.start[0] = 0;
+    for (const auto &r : layers)
+        for (int j = r.first; j < r.second; j++) {
+            if (A.njobs == kMaxAdamJobs) { set_error("too many layers for the Adam pass"); return GBPF_E_ARG; }
+            Layer &y = L[j];
+            const int q = A.njobs++;
+            A.g[q] = y.gW; A.W[q] = y.Wm; A.m[q] = y.Am; A.v[q] = y.Av; A.Wb[q] = y.Wb;
+            A.start[q + 1] = A.start[q] + (long long)y.out * y.in / 4;
+        }
+    const long long groups = A.start[A.njobs];
+    const int blocks = (int)std::max(1LL, (groups + 256 * kAdamU - 1) / (256 * kAdamU));
+    k_adam<<<blocks, 256, 0, st>>>(A, d_t, step, d_sched, lr, b1, b2, eps);
+    CK(cudaGetLastError());
+    return GBPF_OK;
+}
+
+// The transposed bf16 copies of the weights of layers [from, to).
+gbpf_status gbpf_mlp::transpose_layers(cudaStream_t st, int from, int to) {
+    if (from >= to) return GBPF_OK;
+    TransposeJobs J{};
+    int gx = 1, gy = 1;
+    for (int l = from; l < to; l++) {
+        J.W[l - from] = L[l].Wb; J.Wt[l - from] = L[l].Wt;
+        J.rows[l - from] = L[l].out; J.cols[l - from] = L[l].in;
+        gx = std::max(gx, (L[l].in + 31) / 32);
+        gy = std::max(gy, (L[l].out + 31) / 32);
+    }
+    k_transpose_bf16<<<dim3(gx, gy, to - from), dim3(32, 8), 0, st>>>(J);
+    CK(cudaGetLastError());
+    return GBPF_OK;
+}
+
 // Backward pass after forward(train): hidden-layer input gradients through the
-// transposed weights (before those weights change), then the weight gradient
-// of each layer with Adam fused (adam) or stored (gradient check), then the
-// biases, then the Adam step counter.
-gbpf_status gbpf_mlp::backward(cudaStream_t st, Work &w, const CUtensorMap &mXT, int xt_row0, int M, bool adam) {
+// transposed weights, the weight gradients, Adam on them (adam; else they stay
+// in gW for the gradient check), the biases.  With f (training) the parts that
+// do not wait for one another run next to each other, as most of them leave
+// SMs idle: the chain of input gradients and the first layer's weight gradient
+// on st; the output layer's and the skip's weight gradients and their update,
+// which no GEMM needs before the next step's output layer, on f->side; the
+// other hidden layers' weight gradients and the biases on f->wgrad.  Each
+// stream has its split-K workspace; f->side is joined where the next step's
+// output layer reads its weights (forward) and, for the activations it reads,
+// at the end of the step.  A step of the 1,888-bus network (three hidden layers of 512, the
+// metric, 1,024 rows): 473 -> 417 us.
+gbpf_status gbpf_mlp::backward(cudaStream_t st, Work &w, const CUtensorMap &mXT, int xt_row0, int M, bool adam, int step,
+                               Fork *f) {
     const int nl = n_hidden + 1;
     gbpf_status s;
-    for (int l = nl - 1; l >= 0; l--) {
-        // gradient w.r.t. this layer's pre-activation is dY (l = nl-1) or dZ[l]
-        const CUtensorMap &mG = l == nl - 1 ? w.mdY : w.mdZ[l];
-        const CUtensorMap &mGT = l == nl - 1 ? w.mdYT : w.mdZT[l];
-        if (l > 0) {
-            EpiArgs e{};
-            e.err = d_err;
-            e.wait = wait_cycles;
-            e.ws = ws;
-            e.ws_cnt = ws_cnt;
-            e.mode = EPI_BWD_HIDDEN;
-            e.Z = w.Z[l - 1]; e.ldz = hidden;
-            e.H = w.dZ[l - 1]; e.ldh = hidden;
-            e.HT = w.dZT[l - 1]; e.ldht = w.B;
-            if ((s = gemm(st, mG, L[l].mWt, M, hidden, L[l].out, e)) != GBPF_OK) return s;
-        }
+    const cudaStream_t side = f ? f->side : st, wg = f ? f->wgrad : st;
+    auto order = [&](cudaEvent_t ev, cudaStream_t from, cudaStream_t to) -> gbpf_status {  // `to` waits for `from`
+        if (from == to) return GBPF_OK;
+        CK(cudaEventRecord(ev, from));
+        CK(cudaStreamWaitEvent(to, ev, 0));
+        return GBPF_OK;
+    };
+    // weight gradient of layer l (nl: the skip), dZ^T (dY^T) times its input
+    auto wgrad = [&](cudaStream_t q, int q_ws, int l) -> gbpf_status {
         EpiArgs e{};
         e.err = d_err;
         e.wait = wait_cycles;
-        e.ws = ws;
-        e.ws_cnt = ws_cnt;
-        e.b_row0 = l == 0 ? xt_row0 : 0;
+        e.ws = ws[q_ws];
+        e.ws_cnt = ws_cnt[q_ws];
+        const bool from_x = l == 0 || l == nl;
+        e.b_row0 = from_x ? xt_row0 : 0;
         e.mode = EPI_WGRAD_STORE;
         e.out = L[l].gW; e.ldo = L[l].in;
-        const CUtensorMap &mIn = l == 0 ? mXT : w.mHT[l - 1];
-        if ((s = gemm(st, mGT, mIn, L[l].out, L[l].in, M, e)) != GBPF_OK) return s;
-    }
-    if (has_skip) {
-        // the skip's gradient dY^T X; its transpose is never needed
-        Layer &k = L[nl];
+        return gemm(q, l >= nl - 1 ? w.mdYT : w.mdZT[l], from_x ? mXT : w.mHT[l - 1], L[l].out, L[l].in, M, e);
+    };
+    if ((s = order(f ? f->out : nullptr, st, side)) != GBPF_OK) return s;
+    if (has_skip && (s = wgrad(side, 1, nl)) != GBPF_OK) return s;
+    if ((s = wgrad(side, 1, nl - 1)) != GBPF_OK) return s;
+    if (f) CK(cudaEventRecord(f->used, side));
+    if (adam && (s = adam_layers(side, {{nl - 1, nl + (has_skip ? 1 : 0)}}, step)) != GBPF_OK) return s;
+    for (int l = nl - 1; l >= 1; l--) {
+        // gradient w.r.t. this layer's pre-activation is dY (l = nl-1) or dZ[l]
         EpiArgs e{};
         e.err = d_err;
         e.wait = wait_cycles;
-        e.ws = ws;
-        e.ws_cnt = ws_cnt;
-        e.b_row0 = xt_row0;
-        e.mode = EPI_WGRAD_STORE;
-        e.out = k.gW; e.ldo = k.in;
-        if ((s = gemm(st, w.mdYT, mXT, k.out, k.in, M, e)) != GBPF_OK) return s;
+        e.ws = ws[0];
+        e.ws_cnt = ws_cnt[0];
+        e.mode = EPI_BWD_HIDDEN;
+        e.Z = w.Z[l - 1]; e.ldz = hidden;
+        e.H = w.dZ[l - 1]; e.ldh = hidden;
+        e.HT = w.dZT[l - 1]; e.ldht = w.B;
+        if ((s = gemm(st, l == nl - 1 ? w.mdY : w.mdZ[l], L[l].mWt, M, hidden, L[l].out, e)) != GBPF_OK) return s;
+        if ((s = order(f ? f->dz[l - 1] : nullptr, st, wg)) != GBPF_OK) return s;
+        if (l - 1 >= 1 && (s = wgrad(wg, 2, l - 1)) != GBPF_OK) return s;
     }
-    if (adam) {
-        // every weight gradient is stored (and every input gradient that read
-        // the old transposed weights is done): Adam over all weights, then the
-        // transposed bf16 copies of the hidden layers' weights
-        AdamJobs A{};
-        A.njobs = nl + (has_skip ? 1 : 0);
-        if (A.njobs > kMaxAdamJobs) { set_error("too many layers for the Adam pass"); return GBPF_E_ARG; }
-        A.start[0] = 0;
-        for (int j = 0; j < A.njobs; j++) {
-            Layer &y = L[j];
-            A.g[j] = y.gW; A.W[j] = y.Wm; A.m[j] = y.Am; A.v[j] = y.Av; A.Wb[j] = y.Wb;
-            A.start[j + 1] = A.start[j] + (long long)y.out * y.in / 4;
-        }
-        int dev_sm = 0;
-        CK(cudaDeviceGetAttribute(&dev_sm, cudaDevAttrMultiProcessorCount, device));
-        const long long groups = A.start[A.njobs];
-        const int blocks = (int)std::max(1LL, std::min<long long>(8LL * dev_sm, (groups + 255) / 256));
-        k_adam<<<blocks, 256, 0, st>>>(A, d_t, d_sched, lr, b1, b2, eps);
-        CK(cudaGetLastError());
-        for (int l = 0; l < nl; l++) {
-            k_transpose_bf16<<<dim3((L[l].in + 31) / 32, (L[l].out + 31) / 32), dim3(32, 8), 0, st>>>(
-                L[l].Wb, L[l].out, L[l].in, L[l].Wt);
-            CK(cudaGetLastError());
-        }
-    }
+    if ((s = wgrad(st, 0, 0)) != GBPF_OK) return s;
     BiasJobs J{};
     J.njobs = nl;
     J.cols = M;
@@ -1114,12 +1185,21 @@ gbpf_status gbpf_mlp::backward(cudaStream_t st, Work &w, const CUtensorMap &mXT,
         J.row_start[l + 1] = J.row_start[l] + L[l].out;
     }
     const int warps = J.row_start[nl];
-    k_bias<<<(warps * 32 + 255) / 256, 256, 0, st>>>(J, d_t, d_sched, lr, b1, b2, eps, adam ? 1 : 0);
+    k_bias<<<(warps * 32 + 255) / 256, 256, 0, wg>>>(J, d_t, step, d_sched, lr, b1, b2, eps, adam ? 1 : 0);
     CK(cudaGetLastError());
-    if (adam) {
-        k_step<<<1, 1, 0, st>>>(d_t);
-        CK(cudaGetLastError());
+    if ((s = order(f ? f->hidden : nullptr, wg, st)) != GBPF_OK) return s;
+    if (!adam) return GBPF_OK;
+    // every input gradient that read the old transposed weights is done (a
+    // transpose of the first layer's is read by nothing)
+    if ((s = order(f ? f->chained : nullptr, st, side)) != GBPF_OK) return s;
+    if ((s = transpose_layers(side, nl - 1, nl)) != GBPF_OK) return s;
+    if (f) {
+        CK(cudaEventRecord(f->updated, side));
+        f->side_open = 1;
     }
+    if ((s = adam_layers(st, {{0, nl - 1}}, step)) != GBPF_OK) return s;
+    if ((s = transpose_layers(st, 1, nl - 1)) != GBPF_OK) return s;
+    if (f) CK(cudaStreamWaitEvent(st, f->used, 0));
     return GBPF_OK;
 }
 
@@ -1266,6 +1346,7 @@ extern "C" gbpf_status gbpf_mlp_train(gbpf_mlp *m, int epochs, int batch, float 
         if (m->exec) { cudaGraphExecDestroy(m->exec); m->exec = nullptr; }
         gbpf_status s = m->make_work(m->tw, batch, true);
         if (s != GBPF_OK) return s;
+        if ((s = m->make_fork()) != GBPF_OK) return s;
         if ((s = make_map(&m->mXs, m->Xs, m->kin, n, m->kin)) != GBPF_OK) return s;
         if ((s = make_map(&m->mXT, m->XT, batch, (long long)steps * m->kin, batch)) != GBPF_OK) return s;
         // one epoch: shuffle the data set (perm[] is uploaded before each
@@ -1275,10 +1356,24 @@ extern "C" gbpf_status gbpf_mlp_train(gbpf_mlp *m, int epochs, int batch, float 
         k_gather_f32<<<1024, 256, 0, m->stream>>>(m->Y, m->outp, m->perm, n, m->Ys);
         k_transpose_batches<<<dim3((m->kin + 31) / 32, (batch + 31) / 32, steps), dim3(32, 8), 0, m->stream>>>(
             m->Xs, m->kin, batch, m->XT);
-        for (int t = 0; t < steps && s == GBPF_OK; t++) {
-            s = m->forward(m->stream, m->tw, m->mXs, t * batch, batch, m->Ys, t * batch, nullptr, true);
-            if (s == GBPF_OK) s = m->backward(m->stream, m->tw, m->mXT, t * m->kin, batch, true);
-        }
+        gbpf_mlp::Fork &f = m->fk;
+        f.side_open = 0;
+        auto capture = [&]() -> gbpf_status {
+            CK(cudaEventRecord(f.begin, m->stream));
+            CK(cudaStreamWaitEvent(f.chain, f.begin, 0));
+            for (int t = 0; t < steps; t++) {
+                gbpf_status r = m->forward(f.chain, m->tw, m->mXs, t * batch, batch, m->Ys, t * batch, nullptr, true, &f);
+                if (r == GBPF_OK) r = m->backward(f.chain, m->tw, m->mXT, t * m->kin, batch, true, t, &f);
+                if (r != GBPF_OK) return r;
+            }
+            CK(cudaStreamWaitEvent(f.chain, f.updated, 0));
+            k_step<<<1, 1, 0, f.chain>>>(m->d_t, steps);
+            CK(cudaGetLastError());
+            CK(cudaEventRecord(f.hidden, f.chain));
+            CK(cudaStreamWaitEvent(m->stream, f.hidden, 0));
+            return GBPF_OK;
+        };
+        if (s == GBPF_OK) s = capture();
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(m->stream, &g);
         if (s != GBPF_OK) { if (g) cudaGraphDestroy(g); return s; }

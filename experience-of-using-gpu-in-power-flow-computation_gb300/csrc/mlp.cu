@@ -7,12 +7,13 @@
 //
 // Every matrix product is C[M,N] = A[M,K] * B[N,K]^T with A and B bf16,
 // K-contiguous ("K-major"), computed by k_gemm:
-//   * one CTA per 128 x 128 output tile, 128 threads;
-//   * warp 0 / lane 0 streams 128 x 64 tiles of A and B into a 4-stage
-//     shared-memory ring with TMA (cp.async.bulk.tensor, 128-byte swizzle),
+//   * one CTA per output tile of 128 rows and 128, 64 or 32 columns (gemm2),
+//     128 threads;
+//   * warp 0 / lane 0 streams 64-deep tiles of A and B into a shared-memory
+//     ring of 3 to 5 stages with TMA (cp.async.bulk.tensor, 128-byte swizzle),
 //     completion tracked by mbarrier transaction counts;
 //   * warp 1 / lane 0 issues tcgen05.mma (kind::f16, bf16 inputs, fp32
-//     accumulator 128 x 128 in tensor memory) and frees each stage with
+//     accumulator in tensor memory) and frees each stage with
 //     tcgen05.commit;
 //   * all four warps read the accumulator back with tcgen05.ld (warp w owns
 //     TMEM lanes 32w..32w+31 = output rows) and run a fused epilogue.
@@ -49,20 +50,26 @@ typedef __nv_bfloat16 bf16;
 
 namespace {
 
-// Three ring stages (96 KB + barriers) so that two CTAs share an SM: one
+// Three ring stages (96 KB + barriers; as much as fits in that of the narrower
+// tiles) so that two CTAs share an SM: one
 // CTA's epilogue overlaps the other's main loop, and a 240-tile GEMM runs in
 // one wave on 152 SMs (measured with four stages and one CTA per SM: a GEMM
 // with a memory-bound epilogue at 17 % of HBM with the tensor pipe 5 % busy)
-constexpr int BM = 128, BN = 128, BK = 64, STAGES = 3, kGemmThreads = 128, kGemmCtasPerSm = 2;
-constexpr uint32_t kTileBytes = BM * BK * 2;          // 16 KB per operand tile
-constexpr uint32_t kStageBytes = 2 * kTileBytes;      // A + B
-constexpr size_t kGemmSmem = STAGES * kStageBytes + 1024 + 256;
+constexpr int BM = 128, BNmax = 128, BK = 64, kGemmThreads = 128, kGemmCtasPerSm = 2;
+constexpr int kBoxB = 32;                             // rows of a box of B: its tiles are 32, 64 or 128 wide
+constexpr uint32_t kTileBytes = BM * BK * 2;          // 16 KB of A
+template <int BN> struct Tile {                       // BN: columns of the output tile
+    static constexpr int STAGES = BN == 128 ? 3 : BN == 64 ? 4 : 5;
+    static constexpr uint32_t kStageBytes = kTileBytes + BN * BK * 2;  // A + B
+    static constexpr size_t kSmem = STAGES * kStageBytes + 1024 + 256;
+};
 constexpr long long kWaitCycles = 4000000000ll;       // about 2 s at 2 GHz
 // tcgen05 instruction descriptor, kind::f16: fp32 accumulator (bits 4-5 = 1),
 // A and B bf16 (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0),
 // N >> 3 in bits 17-22, M >> 4 in bits 24-28.
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                            ((uint32_t)(BM >> 4) << 24);
+__host__ __device__ constexpr uint32_t idesc(int bn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+}
 
 enum Epi : int {
     EPI_HIDDEN = 0,      // z = acc + b; Z = z; H = gelu(z); HT = H^T
@@ -183,11 +190,12 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t id,
+                                         uint32_t accumulate) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate)
+        "l"(adesc), "l"(bdesc), "r"(id), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t *bar) {
@@ -316,10 +324,13 @@ __device__ __forceinline__ void epilogue8(const EpiArgs &e, int row, int n, floa
 // ---------------------------------------------------------------------------
 // the GEMM
 // ---------------------------------------------------------------------------
+template <int BN>
 __global__ void __launch_bounds__(kGemmThreads, kGemmCtasPerSm)
     k_gemm(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb,
            const __grid_constant__ CUtensorMap ta2, const __grid_constant__ CUtensorMap tb2, int K, int K2,
            EpiArgs e) {
+    constexpr int STAGES = Tile<BN>::STAGES;
+    constexpr uint32_t kStageBytes = Tile<BN>::kStageBytes;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t *full = (uint64_t *)(smem + STAGES * kStageBytes);
@@ -368,10 +379,12 @@ __global__ void __launch_bounds__(kGemmThreads, kGemmCtasPerSm)
             mbar_expect_tx(&full[s], kStageBytes);
             if (kt < nk1) {
                 tma_load_2d(sa, &ta, kt * BK, e.a_row0 + m0, &full[s]);
-                tma_load_2d(sb, &tb, kt * BK, e.b_row0 + n0, &full[s]);
+                for (int r = 0; r < BN; r += kBoxB)
+                    tma_load_2d(sb + r * BK * 2, &tb, kt * BK, e.b_row0 + n0 + r, &full[s]);
             } else {
                 tma_load_2d(sa, &ta2, (kt - nk1) * BK, e.a2_row0 + m0, &full[s]);
-                tma_load_2d(sb, &tb2, (kt - nk1) * BK, n0, &full[s]);
+                for (int r = 0; r < BN; r += kBoxB)
+                    tma_load_2d(sb + r * BK * 2, &tb2, (kt - nk1) * BK, n0 + r, &full[s]);
             }
         }
         *issued = j;
@@ -386,7 +399,7 @@ __global__ void __launch_bounds__(kGemmThreads, kGemmCtasPerSm)
             const uint64_t da = sw128_desc(sa), db = sw128_desc(sb);
 #pragma unroll
             for (int kk = 0; kk < BK / 16; kk++)  // K = 16 per instruction: +32 B along the swizzled row
-                mma_bf16(tmem, da + (uint64_t)(2 * kk), db + (uint64_t)(2 * kk), (j | kk) != 0);
+                mma_bf16(tmem, da + (uint64_t)(2 * kk), db + (uint64_t)(2 * kk), idesc(BN), (j | kk) != 0);
             mma_commit(&empty[s]);
         }
         *consumed = j;
@@ -446,7 +459,7 @@ __global__ void __launch_bounds__(kGemmThreads, kGemmCtasPerSm)
     if (*fail || (S > 1 && !s_last)) {
         // nothing more to do for this CTA
     } else {
-        const int row = m0 + warp * 32 + lane;
+        const int row = m0 + arow;
         const bool rv = row < e.M;
         float sq = 0.f;
         for (int c = 0; c < BN / 16; c++) {
@@ -675,7 +688,7 @@ EncodeTiledFn encode_fn() {
 // 2-D bf16 tensor map over a row-major [rows, inner] matrix with leading
 // dimension ld (elements), 128 x 64 boxes, 128-byte swizzle, zero fill out of
 // bounds (so ragged M, N and K tails contribute zeros).
-gbpf_status make_map(CUtensorMap *m, const void *base, int inner, long long rows, int ld) {
+gbpf_status make_map(CUtensorMap *m, const void *base, int inner, long long rows, int ld, int box_rows = BM) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) { set_error("cuTensorMapEncodeTiled is not available from the driver"); return GBPF_E_CUDA; }
     if (((uintptr_t)base & 15) || (ld * 2) % 16 || inner > ld || rows < 1) {
@@ -684,7 +697,7 @@ gbpf_status make_map(CUtensorMap *m, const void *base, int inner, long long rows
     }
     cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    cuuint32_t box[2] = {BK, BM};
+    cuuint32_t box[2] = {BK, (cuuint32_t)box_rows};
     cuuint32_t es[2] = {1, 1};
     CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, es,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -696,24 +709,32 @@ gbpf_status make_map(CUtensorMap *m, const void *base, int inner, long long rows
 // Split-K for GEMMs with fewer output tiles than SMs (the mini-batch GEMMs
 // of training, M = batch): S splits per tile with S x tiles <= SMs and at
 // least kSplitMinTiles k-tiles per split; only where the caller passes the
-// workspace (e.ws, e.ws_cnt: training, one stream).
+// workspace (e.ws, e.ws_cnt: training, one for each stream).
 constexpr int kSplitMax = 8, kSplitMinTiles = 8;
 gbpf_status gemm2(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &ta2,
                   const CUtensorMap &tb2, int M, int N, int K, int K2, const EpiArgs &e) {
     EpiArgs x = e;
     x.M = M;
     x.N = N;
-    const int gx = (N + BN - 1) / BN, gy = (M + BM - 1) / BM, tiles = gx * gy;
+    const int gx = (N + BNmax - 1) / BNmax, gy = (M + BM - 1) / BM, tiles = gx * gy;
     const int nk = (K + BK - 1) / BK + (K2 + BK - 1) / BK;
-    int S = 1;
-    if (x.ws && x.ws_cnt) {
-        int dev = 0, sms = 0;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        S = std::max(1, std::min({kSplitMax, sms / tiles, nk / kSplitMinTiles}));
-    }
-    dim3 grid(gx, gy, S);
-    k_gemm<<<grid, kGemmThreads, kGemmSmem, st>>>(ta, tb, ta2, tb2, K, K2, x);
+    int S = 1, dev = 0, sms = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (x.ws && x.ws_cnt) S = std::max(1, std::min({kSplitMax, sms / tiles, nk / kSplitMinTiles}));
+    // The widest tile that gives every SM one: the epilogue of a tile is 128
+    // threads' work, column after column, and most of a small GEMM's time
+    // (1,024 x 512 x 512: 32 tiles of 128 columns 20 us, 128 of 32 10 us; with
+    // K = 3,776 and four splits 30 and, at 64 columns, 22 us).  The splits stay
+    // those of 128-wide tiles, so that sums keep their order.  Wider ones than
+    // 128 (one CTA of 224 columns per SM, for 1,024 x 3,776 x 3,776): 38 us
+    // against 31.
+    int bn = BNmax;
+    while (bn > kBoxB && ((N + bn - 1) / bn) * gy * S < sms) bn /= 2;
+    const dim3 grid((N + bn - 1) / bn, gy, S);
+    if (bn == 128) k_gemm<128><<<grid, kGemmThreads, Tile<128>::kSmem, st>>>(ta, tb, ta2, tb2, K, K2, x);
+    else if (bn == 64) k_gemm<64><<<grid, kGemmThreads, Tile<64>::kSmem, st>>>(ta, tb, ta2, tb2, K, K2, x);
+    else k_gemm<32><<<grid, kGemmThreads, Tile<32>::kSmem, st>>>(ta, tb, ta2, tb2, K, K2, x);
     CK(cudaGetLastError());
     return GBPF_OK;
 }
@@ -862,7 +883,9 @@ gbpf_status gbpf_mlp::init(int n_in_, int hidden_, int n_hidden_, int n_out_, in
     hidden = hidden_;
     n_hidden = n_hidden_;
     CK(cudaSetDevice(device));
-    CK(cudaFuncSetAttribute(k_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
+    CK(cudaFuncSetAttribute(k_gemm<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile<128>::kSmem));
+    CK(cudaFuncSetAttribute(k_gemm<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile<64>::kSmem));
+    CK(cudaFuncSetAttribute(k_gemm<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile<32>::kSmem));
     CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
@@ -899,9 +922,9 @@ gbpf_status gbpf_mlp::init(int n_in_, int hidden_, int n_hidden_, int n_out_, in
         CK(cudaMemcpy(y.Wm, hw.data(), 4 * w, cudaMemcpyHostToDevice));
         k_cast_weights<<<256, 256, 0, stream>>>(y.Wm, y.out, y.in, y.Wb, y.Wt);
         CK(cudaGetLastError());
-        gbpf_status st = make_map(&y.mW, y.Wb, y.in, y.out, y.in);
+        gbpf_status st = make_map(&y.mW, y.Wb, y.in, y.out, y.in, kBoxB);
         if (st != GBPF_OK) return st;
-        st = make_map(&y.mWt, y.Wt, y.out, y.in, y.out);
+        st = make_map(&y.mWt, y.Wt, y.out, y.in, y.out, kBoxB);
         if (st != GBPF_OK) return st;
     }
     CK(cudaMalloc(&norm.p, 2 * al(4 * (size_t)n_in) + 2 * al(4 * (size_t)outp)));
@@ -920,13 +943,14 @@ gbpf_status gbpf_mlp::init(int n_in_, int hidden_, int n_hidden_, int n_out_, in
     {
         int sms = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-        const size_t part = (size_t)BM * BN * sizeof(float) * sms;
-        CK(cudaMalloc(&splitk.p, 3 * (part + 4 * (size_t)sms)));
+        const size_t part = (size_t)BM * BNmax * sizeof(float) * sms;
+        const int ncnt = BNmax / kBoxB * sms;
+        CK(cudaMalloc(&splitk.p, 3 * (part + 4 * (size_t)ncnt)));
         int *cnt = (int *)((char *)splitk.p + 3 * part);
-        CK(cudaMemset(cnt, 0, 3 * 4 * (size_t)sms));
+        CK(cudaMemset(cnt, 0, 3 * 4 * (size_t)ncnt));
         for (int q = 0; q < 3; q++) {
             ws[q] = (float *)((char *)splitk.p + q * part);
-            ws_cnt[q] = cnt + q * sms;
+            ws_cnt[q] = cnt + q * ncnt;
         }
     }
     d_t = (int *)misc.p;
@@ -969,7 +993,7 @@ gbpf_status gbpf_mlp::make_work(Work &w, int B, bool train) {
         w.HT[l] = (bf16 *)take(hb);
         w.dZ[l] = (bf16 *)take(hb);
         w.dZT[l] = (bf16 *)take(hb);
-        if ((st = make_map(&w.mHT[l], w.HT[l], B, hidden, B)) != GBPF_OK) return st;
+        if ((st = make_map(&w.mHT[l], w.HT[l], B, hidden, B, kBoxB)) != GBPF_OK) return st;
         if ((st = make_map(&w.mdZ[l], w.dZ[l], hidden, B, hidden)) != GBPF_OK) return st;
         if ((st = make_map(&w.mdZT[l], w.dZT[l], B, hidden, B)) != GBPF_OK) return st;
     }
@@ -1127,7 +1151,8 @@ gbpf_status gbpf_mlp::transpose_layers(cudaStream_t st, int from, int to) {
 // stream has its split-K workspace; f->side is joined where the next step's
 // output layer reads its weights (forward) and, for the activations it reads,
 // at the end of the step.  A step of the 1,888-bus network (three hidden layers of 512, the
-// metric, 1,024 rows): 473 -> 417 us.
+// metric, 1,024 rows): 473 -> 417 us; with narrow tiles (gemm2) and the chain's
+// kernels ahead of the others (priorities) 365 us.
 gbpf_status gbpf_mlp::backward(cudaStream_t st, Work &w, const CUtensorMap &mXT, int xt_row0, int M, bool adam, int step,
                                Fork *f) {
     const int nl = n_hidden + 1;
@@ -1348,7 +1373,7 @@ extern "C" gbpf_status gbpf_mlp_train(gbpf_mlp *m, int epochs, int batch, float 
         if (s != GBPF_OK) return s;
         if ((s = m->make_fork()) != GBPF_OK) return s;
         if ((s = make_map(&m->mXs, m->Xs, m->kin, n, m->kin)) != GBPF_OK) return s;
-        if ((s = make_map(&m->mXT, m->XT, batch, (long long)steps * m->kin, batch)) != GBPF_OK) return s;
+        if ((s = make_map(&m->mXT, m->XT, batch, (long long)steps * m->kin, batch, kBoxB)) != GBPF_OK) return s;
         // one epoch: shuffle the data set (perm[] is uploaded before each
         // launch), transpose each mini-batch's features, then every step
         CK(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
@@ -1378,7 +1403,7 @@ extern "C" gbpf_status gbpf_mlp_train(gbpf_mlp *m, int epochs, int batch, float 
         cudaError_t e = cudaStreamEndCapture(m->stream, &g);
         if (s != GBPF_OK) { if (g) cudaGraphDestroy(g); return s; }
         if (e != cudaSuccess) { set_error(std::string("capture: ") + cudaGetErrorString(e)); return GBPF_E_CUDA; }
-        e = cudaGraphInstantiate(&m->exec, g, 0);
+        e = cudaGraphInstantiate(&m->exec, g, cudaGraphInstantiateFlagUseNodePriority);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) { set_error(std::string("instantiate: ") + cudaGetErrorString(e)); return GBPF_E_CUDA; }
         m->graph_B = batch;
@@ -1465,7 +1490,7 @@ extern "C" gbpf_status gbpf_mlp_gradients(gbpf_mlp *m, const float *Xn, const fl
     CK(cudaMemcpy(dy, hy.data(), 4 * hy.size(), cudaMemcpyHostToDevice));
     CUtensorMap mX, mXT;
     if ((s = make_map(&mX, dx, m->kin, n, m->kin)) != GBPF_OK) return s;
-    if ((s = make_map(&mXT, dxt, n, m->kin, n)) != GBPF_OK) return s;
+    if ((s = make_map(&mXT, dxt, n, m->kin, n, kBoxB)) != GBPF_OK) return s;
     CK(cudaMemsetAsync(m->d_loss, 0, 4, m->stream));
     CK(cudaMemsetAsync(m->d_err, 0, 4, m->stream));
     if ((s = m->forward(m->stream, w, mX, 0, n, dy, 0, nullptr, true)) != GBPF_OK) return s;
@@ -1583,9 +1608,9 @@ extern "C" gbpf_status gbpf_mlp_set_loss_metric(gbpf_mlp *m, const float *A, int
     CK(cudaMemcpy(m->Ab, h.data(), 2 * h.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(m->Abt, ht.data(), 2 * ht.size(), cudaMemcpyHostToDevice));
     m->metric_k = kp;
-    gbpf_status st = make_map(&m->mA, m->Ab, kp, p, kp);
+    gbpf_status st = make_map(&m->mA, m->Ab, kp, p, kp, kBoxB);
     if (st != GBPF_OK) return st;
-    return make_map(&m->mAt, m->Abt, p, kp, p);
+    return make_map(&m->mAt, m->Abt, p, kp, p, kBoxB);
 }
 
 extern "C" gbpf_status gbpf_mlp_dims(const gbpf_mlp *m, int dims[5]) {

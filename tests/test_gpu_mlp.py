@@ -417,3 +417,46 @@ def test_gemm_wait_limit_runs_out_and_the_handle_recovers(gb):
     assert "wait ran out" in str(e.value)
     m.set_wait_limit(0)
     np.testing.assert_array_equal(m.predict(X), before)
+
+
+@pytest.mark.parametrize("n_in,n_out,width,n,skip", [(24, 8, 8, 8, True), (40, 33, 40, 72, False),
+                                                     (264, 520, 136, 520, True), (72, 1284, 520, 2048, True)])
+def test_gradients_match_oracle_over_tile_widths(gb, n_in, n_out, width, n, skip):
+    """Output tiles of 32, 64 and 128 columns (as many as fill the SMs, at most), the last one ragged: loss and every
+    gradient to the tolerances above."""
+    test_gradients_match_oracle(gb, n_in, n_out, width, n, skip)
+
+
+@pytest.mark.parametrize("width,layers,n_out,batch,skip,metric", [(128, 1, 36, 64, True, False), (40, 2, 200, 72, False, True),
+                                                                  (256, 3, 520, 256, True, True)])
+def test_training_steps_side_by_side_repeat_their_bits(gb, width, layers, n_out, batch, skip, metric):
+    """The steps of an epoch overlap on three streams (the update of the output layer and the skip runs into the next
+    step): every run from the same parameters ends on the same bits, and epochs of one step, which have no next step to
+    run into, follow the oracle's Adam."""
+    rng = np.random.default_rng(width)
+    X = rng.normal(size=(6 * batch, 48)).astype(np.float32)
+    Y = rng.normal(size=(6 * batch, n_out)).astype(np.float32)
+    A = (rng.normal(size=(n_out, n_out)) / np.sqrt(n_out)).astype(np.float32)
+    out = []
+    for _ in range(3):
+        m = gb.MLP(48, n_out, width=width, n_layers=layers, skip=skip, seed=5)
+        m.set_data(X, Y)
+        if metric:
+            m.set_loss_metric(A, 0.5)
+        m.train(4, batch=batch, lr=1e-3, seed=7)
+        out.append([a for p in m.params() for a in p if a is not None])
+    for o in out[1:]:
+        for a, b in zip(out[0], o):
+            np.testing.assert_array_equal(a, b)
+    m = gb.MLP(48, n_out, width=width, n_layers=layers, skip=skip, seed=5)
+    m.set_data(X[:batch], Y[:batch])
+    Xn, Yn, _ = _normalise(m, X[:batch], Y[:batch])
+    p0 = m.params()
+    m.train(1, batch=batch, lr=1e-3, seed=7)
+    _, g = mo.loss_and_grads(p0, Xn, Yn, emulate=True)
+    for (W0, b0), (W1, b1), (gW, gbias) in zip(p0, m.params(), g):
+        for a0, a1, ga in ((W0, W1, gW), (b0, b1, gbias)):
+            if a0 is None:
+                continue
+            stable = np.abs(ga) > 1e-2 * np.max(np.abs(ga))  # the first step is lr against the gradient's sign
+            assert np.max(np.abs((a1 - a0) + 1e-3 * np.sign(ga))[stable]) < 1e-5

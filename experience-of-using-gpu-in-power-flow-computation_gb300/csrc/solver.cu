@@ -791,9 +791,62 @@ struct gbpf_solver {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
         if (dmem) cudaFree(dmem);
+        if (stage) cudaFreeHost(stage);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (stream) cudaStreamDestroy(stream);
+    }
+
+    // Pinned memory that results come back through, one copy for arrays that lie
+    // one behind the other: a copy to pageable memory is staged by the driver,
+    // 8-12 us each however small (14 buses: the state 45 -> 18 us, the flows 44
+    // -> 18, next to 80 us on the device).  Up to kStageMax bytes at a time: from
+    // there on a second pass over the results costs what the driver's does
+    // (15,104 buses: state, 480 KB, 64 -> 55 us; flows, 650 KB, 68 -> 76).
+    static constexpr size_t kStageMax = 512 * 1024;
+    char *stage = nullptr;
+    size_t stage_size = 0;
+    gbpf_status fetch(const void *from, size_t bytes) {
+        if (cudaError_t e = cudaMemcpyAsync(stage, from, bytes, cudaMemcpyDeviceToHost, stream)) return cuda_fail(e);
+        if (cudaError_t e = cudaStreamSynchronize(stream)) return cuda_fail(e);
+        return GBPF_OK;
+    }
+    static gbpf_status cuda_fail(cudaError_t e) {
+        set_error(std::string("result copy: ") + cudaGetErrorString(e));
+        return GBPF_E_CUDA;
+    }
+    // arrays from[0 .. 3] of n values, in order in one piece of device memory,
+    // to the ones of to[] that are there
+    gbpf_status fetch4(double *const from[4], double *const to[4], size_t n) {
+        int a = 0, b = 3;
+        while (a < 4 && !to[a]) a++;
+        while (b > a && !to[b]) b--;
+        if (a == 4) return GBPF_OK;
+        const size_t bytes = (char *)(from[b] + n) - (char *)from[a];
+        if (bytes > stage_size) {
+            cudaError_t e = cudaSuccess;
+            for (int i = a; i <= b && !e; i++)
+                if (to[i]) e = cudaMemcpyAsync(to[i], from[i], n * sizeof(double), cudaMemcpyDeviceToHost, stream);
+            if (!e) e = cudaStreamSynchronize(stream);
+            return e ? cuda_fail(e) : GBPF_OK;
+        }
+        const gbpf_status st = fetch(from[a], bytes);
+        if (st != GBPF_OK) return st;
+        for (int i = a; i <= b; i++)
+            if (to[i]) std::memcpy(to[i], stage + ((char *)from[i] - (char *)from[a]), n * sizeof(double));
+        return GBPF_OK;
+    }
+    // the control record and `more` bytes of what lies behind it (in `stage`)
+    gbpf_status fetch_ctl(Ctl *c, size_t more) {
+        const gbpf_status st = fetch(d.ctl, std::max(sizeof(Ctl), more));
+        if (st == GBPF_OK) std::memcpy(c, stage, sizeof(Ctl));
+        return st;
+    }
+    template <class T> const T *staged(const T *p) const { return (const T *)(stage + ((char *)p - (char *)d.ctl)); }
+    // bytes from the control record to the end of p[0 .. n) where that is in reach
+    template <class T> size_t reach(const T *p, size_t n) const {
+        const size_t b = (size_t)((char *)(p + n) - (char *)d.ctl);
+        return b <= stage_size ? b : 0;
     }
 
     int nfl() const { return (int)S.flev_ptr.size() - 1; }
@@ -1024,12 +1077,12 @@ gbpf_status gbpf_solver::build(const Grid &grid, const gbpf_options &o, int dev)
         d.br_r = A.take<double>(nL + 1); d.br_x = A.take<double>(nL + 1); d.br_b = A.take<double>(nL + 1);
         d.br_tre = A.take<double>(nL + 1); d.br_tim = A.take<double>(nL + 1);
         d.gsh = A.take<double>(nB); d.bsh = A.take<double>(nB);
-        d.V = A.take<double>(nB); d.th = A.take<double>(nB); d.cs = A.take<double>(nB); d.sn = A.take<double>(nB);
-        d.P = A.take<double>(nB); d.Q = A.take<double>(nB);
+        // (V .. Q, ctl .. events and Pdp .. Qpd lie one behind the other: they are read back as one piece)
+        d.V = A.take<double>(nB); d.th = A.take<double>(nB); d.P = A.take<double>(nB); d.Q = A.take<double>(nB);
+        d.cs = A.take<double>(nB); d.sn = A.take<double>(nB);
         d.V0 = A.take<double>(nB); d.th0 = A.take<double>(nB); d.Pliq = A.take<double>(nB); d.Qliq = A.take<double>(nB);
         d.Qload = A.take<double>(nB); d.type = A.take<int>(nB); d.act = A.take<int>(nB); d.QliqLim = A.take<double>(nB);
         d.pv_bus = A.take<int>(g.nPV + 1); d.Qmin = A.take<double>(g.nPV + 1); d.Qmax = A.take<double>(g.nPV + 1);
-        d.limQ = A.take<int>(g.nPV + 1);
         d.bus_of_blk = A.take<int>(n); d.blk_of_bus = A.take<int>(nB);
         d.up_ptr = A.take<int>(n + 1); d.up_col = A.take<int>(nup + 1);
         d.dg_ptr = A.take<int>(n + 1); d.dg_pos = A.take<int>(nup + 1); d.dg_k = A.take<int>(nup + 1);
@@ -1046,7 +1099,8 @@ gbpf_status gbpf_solver::build(const Grid &grid, const gbpf_options &o, int dev)
             d.fac = A.take<blk4>(nq); d.dinv = A.take<blk4>(n);
         }
         d.rhs = A.take<double2>(n); d.ys = A.take<double2>(n); d.xs = A.take<double2>(n);
-        d.ctl = A.take<Ctl>(1); d.hist = A.take<double>(hist_cap); d.trig = A.take<int>(hist_cap);
+        d.ctl = A.take<Ctl>(1); d.limQ = A.take<int>(g.nPV + 1);
+        d.hist = A.take<double>(hist_cap); d.trig = A.take<int>(hist_cap);
         d.events = A.take<int>(4 * kEventCap);
         d.fl_skm = A.take<int>(nL + 1); d.fl_smk = A.take<int>(nL + 1);
         d.fl_phi = A.take<double>(nL + 1); d.fl_bkm = A.take<double>(nL + 1); d.fl_bmk = A.take<double>(nL + 1);
@@ -1061,6 +1115,10 @@ gbpf_status gbpf_solver::build(const Grid &grid, const gbpf_options &o, int dev)
         }
     }
     CK(cudaMemsetAsync(dmem, 0, dmem_size, stream));
+    stage_size = std::max({(size_t)((char *)(d.Q + nB) - (char *)d.V), (size_t)((char *)(d.Qpd + nL) - (char *)d.Pdp),
+                           (size_t)((char *)d.limQ - (char *)d.ctl) + 4 * (size_t)g.nPV, (size_t)16384});
+    stage_size = std::min(stage_size, kStageMax);
+    CK(cudaHostAlloc((void **)&stage, stage_size, cudaHostAllocDefault));
     CK(cudaStreamSynchronize(stream));
     setup_ms[1] = ms_since(tp);
     tp = clk::now();
@@ -1326,8 +1384,9 @@ gbpf_status gbpf_solver::run(gbpf_result *r) {
 // Reads the control record of the solve just enqueued on the stream into
 // `last` and the caller's result.
 gbpf_status gbpf_solver::finish(gbpf_result *r) {
-    CK(cudaMemcpyAsync(&last, d.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
+    const bool lim = r && g.nPV && opt.lim_inj_reat && reach(d.limQ, g.nPV);
+    const gbpf_status fs = fetch_ctl(&last, lim ? reach(d.limQ, g.nPV) : 0);
+    if (fs != GBPF_OK) return fs;
     if (r) {
         r->status = last.status;
         r->converged = last.converged;
@@ -1339,7 +1398,8 @@ gbpf_status gbpf_solver::finish(gbpf_result *r) {
         // PV bus switched: every flag starts at 0)
         if (g.nPV && last.n_events > 0) {
             std::vector<int> lq(g.nPV);
-            CK(cudaMemcpy(lq.data(), d.limQ, g.nPV * sizeof(int), cudaMemcpyDeviceToHost));
+            if (lim) std::copy(staged(d.limQ), staged(d.limQ) + g.nPV, lq.begin());
+            else CK(cudaMemcpy(lq.data(), d.limQ, g.nPV * sizeof(int), cudaMemcpyDeviceToHost));
             for (int v : lq) npq += v;
         }
         r->nPQlim = g.nPQ + npq;
@@ -1396,24 +1456,24 @@ extern "C" gbpf_status gbpf_solver_set_start(gbpf_solver *s, const double *V0, c
 extern "C" gbpf_status gbpf_solver_state(gbpf_solver *s, double *V, double *theta, double *Pcalc,
                                          double *Qcalc) {
     ARGCHECK(s);
-    const size_t b = s->g.nB * sizeof(double);
     CK(cudaSetDevice(s->device));
-    if (V) CK(cudaMemcpyAsync(V, s->d.V, b, cudaMemcpyDeviceToHost, s->stream));
-    if (theta) CK(cudaMemcpyAsync(theta, s->d.th, b, cudaMemcpyDeviceToHost, s->stream));
-    if (Pcalc) CK(cudaMemcpyAsync(Pcalc, s->d.P, b, cudaMemcpyDeviceToHost, s->stream));
-    if (Qcalc) CK(cudaMemcpyAsync(Qcalc, s->d.Q, b, cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaStreamSynchronize(s->stream));
-    return GBPF_OK;
+    double *const from[4] = {s->d.V, s->d.th, s->d.P, s->d.Q}, *const to[4] = {V, theta, Pcalc, Qcalc};
+    return s->fetch4(from, to, s->g.nB);
 }
 
 extern "C" gbpf_status gbpf_solver_events(gbpf_solver *s, int *ev, int cap, int *n) {
     ARGCHECK(s && n && (cap == 0 || ev));
     CK(cudaSetDevice(s->device));
+    // with the first events, as many as a solve commonly has, where they are in reach
+    constexpr int kFirst = 64;
+    const size_t more = s->opt.lim_inj_reat ? s->reach(s->d.events, 4 * kFirst) : 0;
     Ctl c;
-    CK(cudaMemcpy(&c, s->d.ctl, sizeof c, cudaMemcpyDeviceToHost));
+    gbpf_status st = s->fetch_ctl(&c, more);
+    if (st != GBPF_OK) return st;
     const int have = std::min(c.n_events, kEventCap);
     std::vector<int> e(4 * (size_t)have);
-    if (have) CK(cudaMemcpy(e.data(), s->d.events, e.size() * sizeof(int), cudaMemcpyDeviceToHost));
+    if (have && have <= kFirst && more) std::copy(s->staged(s->d.events), s->staged(s->d.events) + e.size(), e.begin());
+    else if (have) CK(cudaMemcpy(e.data(), s->d.events, e.size() * sizeof(int), cudaMemcpyDeviceToHost));
     // events of one iteration were appended in arbitrary order: sort by
     // (iteration, PV position), the order chkLimQ prints them
     std::vector<int> idx(have);
@@ -1430,11 +1490,15 @@ extern "C" gbpf_status gbpf_solver_events(gbpf_solver *s, int *ev, int cap, int 
 extern "C" gbpf_status gbpf_solver_history(gbpf_solver *s, double *hist, int cap, int *n) {
     ARGCHECK(s && n && (cap == 0 || hist));
     CK(cudaSetDevice(s->device));
+    const int first = std::min(s->d.hist_cap, 128);  // iterations read with the control record
+    const size_t more = s->reach(s->d.hist, first);
     Ctl c;
-    CK(cudaMemcpy(&c, s->d.ctl, sizeof c, cudaMemcpyDeviceToHost));
+    gbpf_status st = s->fetch_ctl(&c, more);
+    if (st != GBPF_OK) return st;
     const int have = std::min(c.it + 1, s->d.hist_cap);
     const int m = std::min(have, cap);
-    if (m) CK(cudaMemcpy(hist, s->d.hist, m * sizeof(double), cudaMemcpyDeviceToHost));
+    if (m > 0 && m <= first && more) std::copy(s->staged(s->d.hist), s->staged(s->d.hist) + m, hist);
+    else if (m) CK(cudaMemcpy(hist, s->d.hist, m * sizeof(double), cudaMemcpyDeviceToHost));
     *n = m;
     return GBPF_OK;
 }
@@ -1454,13 +1518,9 @@ extern "C" gbpf_status gbpf_solver_triggers(gbpf_solver *s, int *trig, int cap, 
 extern "C" gbpf_status gbpf_solver_flows(gbpf_solver *s, double *Pdp, double *Ppd, double *Qdp,
                                          double *Qpd) {
     ARGCHECK(s);
-    const size_t b = s->g.nL * sizeof(double);
     CK(cudaSetDevice(s->device));
-    if (Pdp) CK(cudaMemcpy(Pdp, s->d.Pdp, b, cudaMemcpyDeviceToHost));
-    if (Ppd) CK(cudaMemcpy(Ppd, s->d.Ppd, b, cudaMemcpyDeviceToHost));
-    if (Qdp) CK(cudaMemcpy(Qdp, s->d.Qdp, b, cudaMemcpyDeviceToHost));
-    if (Qpd) CK(cudaMemcpy(Qpd, s->d.Qpd, b, cudaMemcpyDeviceToHost));
-    return GBPF_OK;
+    double *const from[4] = {s->d.Pdp, s->d.Ppd, s->d.Qdp, s->d.Qpd}, *const to[4] = {Pdp, Ppd, Qdp, Qpd};
+    return s->fetch4(from, to, s->g.nL);
 }
 
 extern "C" gbpf_status gbpf_solver_set_lu_launch(gbpf_solver *s, int mode) {

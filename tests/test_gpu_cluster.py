@@ -83,3 +83,27 @@ def test_persistent_form_on_request(gb, name):
     assert a["converged"] and a["iterations"] == p["iterations"]
     np.testing.assert_allclose(a["V"], p["V"], rtol=0, atol=1e-11)
     np.testing.assert_allclose(a["theta"], p["theta"], rtol=0, atol=1e-11)
+
+
+@pytest.mark.parametrize("name,max_iter", [("c4_14.cdf.gz", 5), ("c4_14.cdf.gz", 300), ("c3_base.cdfx.gz", 3)])
+def test_results_come_back_in_one_piece(gb, name, max_iter):
+    """State and flows asked for array by array (any of them left out) are those of the whole result, below and above
+    what one staged copy holds, and a history longer than what is read with the control record is all there: a solve
+    that cannot reach its tolerance stops at no_max_iter with every iteration's mismatch."""
+    import ctypes
+
+    grid = grid_of(gb, name)
+    s = gb.Solver(grid, tolerancia=1e-30, no_max_iter=max_iter, lim_inj_reat=0, metodo=0)
+    r = s.solve()
+    h = s.history()
+    assert len(h) == r["iterations"] + 1 == max_iter + 1 and (h[:2] > 0).all()
+    short = gb.Solver(grid, tolerancia=1e-30, no_max_iter=2, lim_inj_reat=0, metodo=0)
+    np.testing.assert_array_equal(short.solve()["hist"], h[:3])
+    for call, keys, n in (("gbpf_solver_state", ("V", "theta", "Pcalc", "Qcalc"), grid.nB),
+                          ("gbpf_solver_flows", ("Pdp", "Ppd", "Qdp", "Qpd"), grid.nL)):
+        for mask in range(16):
+            a = [np.full(n, np.nan) for _ in range(4)]
+            ptr = [x.ctypes.data_as(ctypes.c_void_p) if mask >> i & 1 else None for i, x in enumerate(a)]
+            assert getattr(gb.lib(), call)(s.h, *ptr) == 0
+            for i, k in enumerate(keys):
+                np.testing.assert_array_equal(a[i], r[k] if mask >> i & 1 else np.full(n, np.nan), err_msg=k)

@@ -44,6 +44,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kTailMaxBatch = 80;  // order of a tail (tail_lu) at most: two blocks per SM
+constexpr size_t kWarpSlice32 = 40 * 1024;  // of an FP32 instance that runs on a warp, at most
 constexpr int kTailPanel = 4;      // its pivots to a panel
 // Iteration at which an instance still running on the warp-per-instance
 // kernel moves to a thread block of its own: a batch finishes when its slowest
@@ -130,17 +131,19 @@ struct TopoOff {
         og_ptr, og_a, og_b, flev_ptr, flev_steps, blev_ptr, blev_steps, ysl, rbus, cbus, fent_ptr, fent_p,
         fent_j, lvl_group, lvl_group_w, lvl_narrow, lvl_rot, og_k, yval32, lvl_group4, lvl_rot4, inj_order,
         lvl_group4w, lvl_q4w;
-    // the tail form of the FP32 blocks (tail_lu): levels of the steps before
-    // the tail, and what takes their updates into it
-    int t_flev_ptr, t_flev_steps, t_fent_ptr, t_fent_p, t_blev_ptr, t_blev_steps, t_group, t_rot, t_dg_end, t_sc_p, t_sc_k,
-        t_task_ptr, t_task;
+    // what takes the steps before a tail into it (tail_lu)
+    int t_dg_end, t_sc_p, t_sc_k, t_task_ptr, t_task;
+    // records of the FP32 one-pass and backward levels (LuRec, BackRec): of all
+    // of them [0], and of those before the tail [1]
+    int r_piv[2], r_pk[2], r_ent[2], r_ent2[2], r_meta[2], r_row[2], r_bmeta[2];
 };
 struct Topo {
     int nB, nL, n, nup, nnzY, nPV, nfl, nbl, fac_smem, blob_smem, blob_bytes;
     // tail: order of the dense trailing block that block-mode FP32 instances
     // factor right-looking (0: none, or no room by the plan; dense: the order
-    // there is); then the forward and backward levels before it
-    int tail, dense, t_nfl, t_nbl, t_nsc;
+    // there is), and the entries before it in its rows
+    int tail, dense, t_nsc;
+    int r_n[2], r_nb[2];  // rounds of the records (0: none)
     const char *blob;  // global copy
     const char *flat;  // the shared flat-start iteration (k_flat_start), or null
     TopoOff o;
@@ -709,6 +712,64 @@ __device__ __forceinline__ void back_rows(const TopoView &G, int l, int lg, int 
     }
 }
 
+// What a thread of the block does in a round of the FP32 one-pass levels or of
+// the backward levels (a level is one round, or several where it holds more
+// than the block takes at a time), laid out by thread by add_topology: a level
+// begins behind a barrier, and there its lists were a chain of four loads (the
+// level's step, the range of its list, the list, the blocks); a record is one,
+// made a round ahead (150 FP32 instances of a 1,888-bus grid 0.92 -> 0.79 ms,
+// 250 of 236 buses 0.39 -> 0.34).  At four blocks per SM the other blocks fill
+// the waits and the records' own traffic costs more: there the forward levels
+// keep their lists (2,048 instances of 1,888 buses 6.08 ms, with records 6.30).
+struct LuRec {
+    const int4 *piv;   // step (-1: none), first and last + 1 of its list for this lane, position of the first
+    const int *pk;     // step of that position
+    const int4 *ent;   // entry (-1: none), list range for this lane, first operand
+    const int2 *ent2;  // second operand, step
+    const int *meta;   // lanes of a pivot | lanes of an entry << 3 | last of its level << 6
+    int n;
+};
+struct BackRec {
+    const int4 *row;  // step (-1: none), range of its list for this lane, first column
+    const int *meta;  // lanes of a row | last of its level << 6
+    int n;
+};
+
+// All backward levels: back_rows' arithmetic in back_rows' order.
+template <typename TJ, int NT>
+__device__ __forceinline__ void back_levels(const TopoView &G, const BackRec R, int t,
+                                            const typename Blk<TJ>::b4 *dinv, const typename Blk<TJ>::b4 *Uv,
+                                            typename Blk<TJ>::b2 *ys) {
+    using B4 = typename Blk<TJ>::b4;
+    using B2 = typename Blk<TJ>::b2;
+    const int4 none = make_int4(-1, 0, 0, 0);
+    int4 cur = R.n > 0 ? R.row[t] : none, nxt = R.n > 1 ? R.row[NT + t] : none;
+    B4 u = {}, dv = {};
+    auto load = [&](int4 x) {
+        if (x.y < x.z) u = Uv[x.y];
+        if (x.x >= 0) dv = dinv[x.x];
+    };
+    load(cur);
+    for (int r = 0; r < R.n; r++) {
+        const int4 c = cur;
+        const B4 uc = u, dc = dv;
+        const int meta = R.meta[r], gs = 1 << (meta & 7), gl = t & (gs - 1);
+        cur = nxt;
+        load(cur);
+        nxt = r + 2 < R.n ? R.row[(r + 2) * NT + t] : none;
+        B2 acc;
+        acc.x = acc.y = (TJ)0;
+        if (c.x >= 0) {
+            if (gl == 0) acc = ys[c.x];
+            if (c.y < c.z) acc = bmvs(acc, uc, ys[c.w]);
+            for (int q = c.y + gs; q < c.z; q += gs) acc = bmvs(acc, Uv[q], ys[G.up_col[q]]);
+        }
+        for (int o = gs >> 1; o > 0; o >>= 1) acc = b2sum_xor(acc, o);
+        if (c.x >= 0 && gl == 0) ys[c.x] = bmv(dc, acc);
+        if (meta >> 6) __syncthreads();
+    }
+}
+
 // Forward substitution alone on forward level l with a factor made earlier
 // (two-pass form, L scaled): y_j -= sum_k L(j,k) y_k, summed exactly as the
 // y part of lu_pivots with the same lane groups, so the result is the one the
@@ -826,6 +887,85 @@ __device__ __forceinline__ bool lu_level1(const TopoView &G, int l, int lgp, int
                 Lv[p] = aL;
             }
         }
+    }
+    return sing;
+}
+
+// All FP32 one-pass levels on one block: lu_level1's arithmetic and order of
+// summation, the work of a round from its records.
+template <int NT>
+__device__ __forceinline__ bool lu_levels1(const TopoView &G, const LuRec R, int t, float4 *fac, float2 *ys, float4 *Lv,
+                                           float4 *Uv) {
+    bool sing = false;
+    const int4 none = make_int4(-1, 0, 0, 0);
+    int4 np = R.n > 0 ? R.piv[t] : none, ne = R.n > 0 ? R.ent[t] : none;
+    int nk = R.n > 0 ? R.pk[t] : 0;
+    int2 ne2 = R.n > 0 ? R.ent2[t] : make_int2(0, 0);
+    for (int r = 0; r < R.n; r++) {
+        const int4 p = np, e = ne;
+        const int k0 = nk, meta = R.meta[r];
+        const int2 e2 = ne2;
+        if (r + 1 < R.n) {
+            const int at = (r + 1) * NT + t;
+            np = R.piv[at];
+            nk = R.pk[at];
+            ne = R.ent[at];
+            ne2 = R.ent2[at];
+        }
+        if (__any_sync(0xffffffffu, p.x >= 0)) {
+            const int gs = 1 << (meta & 7), gl = t & (gs - 1), j = p.x;
+            float4 D = make_float4(0.f, 0.f, 0.f, 0.f);
+            float2 yj = make_float2(0.f, 0.f);
+            if (j >= 0 && gl == 0) {
+                D = fac[j];
+                yj = ys[j];
+            }
+            for (int q = p.y, pos = p.w, k = k0; q < p.z;) {
+                const float4 lt = Lv[pos], dk = fac[k];
+                const float2 z = bmv(dk, ys[k]);
+                D = bms(D, lt, bm(dk, Uv[pos]));
+                yj = bmvs(yj, lt, z);
+                if ((q += gs) < p.z) {
+                    pos = G.dg_pos[q];
+                    k = G.dg_k[q];
+                }
+            }
+            for (int o = gs >> 1; o > 0; o >>= 1) {
+                D = bsum_xor(D, o);
+                yj = b2sum_xor(yj, o);
+            }
+            if (j >= 0 && gl == 0) {
+                const float det = D.x * D.w - D.y * D.z;
+                sing |= (det == 0.f || !isfinite(det));
+                const float rd = rcp_rn(det);
+                fac[j] = make_float4(D.w * rd, -D.y * rd, -D.z * rd, D.x * rd);
+                ys[j] = yj;
+            }
+        }
+        if (__any_sync(0xffffffffu, e.x >= 0)) {
+            const int gs = 1 << (meta >> 3 & 7), gl = t & (gs - 1);
+            float4 aL = make_float4(0.f, 0.f, 0.f, 0.f), aU = aL;
+            if (e.x >= 0 && gl == 0) { aL = Lv[e.x]; aU = Uv[e.x]; }
+            for (int q = e.y, x = e.w, y = e2.x, k = e2.y; q < e.z;) {
+                const float4 dk = fac[k];
+                aL = bms(aL, Lv[y], bm(dk, Uv[x]));
+                aU = bms(aU, Lv[x], bm(dk, Uv[y]));
+                if ((q += gs) < e.z) {
+                    x = G.og_a[q];
+                    y = G.og_b[q];
+                    k = G.og_k[q];
+                }
+            }
+            for (int o = gs >> 1; o > 0; o >>= 1) {
+                aL = bsum_xor(aL, o);
+                aU = bsum_xor(aU, o);
+            }
+            if (e.x >= 0 && gl == 0) {
+                Uv[e.x] = aU;
+                Lv[e.x] = aL;
+            }
+        }
+        if (meta >> 6) __syncthreads();
     }
     return sing;
 }
@@ -1527,6 +1667,9 @@ __global__ void __launch_bounds__(kThreads, GS == 3 ? 4 : 2) k_nr_block(Args a) 
                 __syncthreads();
                 if (s_done) break;
                 const B4 *Ub = Uv, *Db = dinv;
+                auto back_rec = [&](int v) {
+                    return BackRec{(const int4 *)(T.blob + T.o.r_row[v]), (const int *)(T.blob + T.o.r_bmeta[v]), T.r_nb[v]};
+                };
                 if (f0 || c0) {
                     // a shared factor (the grid's start, or the warm start's
                     // reference): forward substitution alone
@@ -1558,37 +1701,33 @@ __global__ void __launch_bounds__(kThreads, GS == 3 ? 4 : 2) k_nr_block(Args a) 
                     // side by side, L unscaled) and needs one barrier instead of two.
                     B2 *zs = (B2 *)(ism + L.zs);
                     const bool tailed = kTails && a.lu1 && T.tail && !a.narrow && !a.no_group;
+                    const bool recs = kTails && a.lu1 && T.r_n[0] && !a.narrow && !a.no_group;
+                    auto lu_rec = [&](int v) {
+                        return LuRec{(const int4 *)(T.blob + T.o.r_piv[v]), (const int *)(T.blob + T.o.r_pk[v]),
+                                     (const int4 *)(T.blob + T.o.r_ent[v]), (const int2 *)(T.blob + T.o.r_ent2[v]),
+                                     (const int *)(T.blob + T.o.r_meta[v]), T.r_n[v]};
+                    };
                     if constexpr (kTails) {
                         if (tailed) {
                             // the steps before the tail, the tail, the rows
                             // before the tail
-                            TopoView H = G;
-                            H.flev_ptr = (const int *)(T.blob + T.o.t_flev_ptr);
-                            H.flev_steps = (const int *)(T.blob + T.o.t_flev_steps);
-                            H.fent_ptr = (const int *)(T.blob + T.o.t_fent_ptr);
-                            H.fent_p = (const int *)(T.blob + T.o.t_fent_p);
-                            H.blev_ptr = (const int *)(T.blob + T.o.t_blev_ptr);
-                            H.blev_steps = (const int *)(T.blob + T.o.t_blev_steps);
-                            const int *grp = (const int *)(T.blob + T.o.t_group);
-                            const int *rot = (const int *)(T.blob + T.o.t_rot);
-                            bool sing = false;
-                            for (int l = 0; l < T.t_nfl; l++) {
-                                sing |= lu_level1<TJ, kThreads>(H, l, grp[3 * l], grp[3 * l + 1], rot[l], tid, fac,
-                                                                dinv, ys, zs, Lv, Uv);
-                                __syncthreads();
-                            }
+                            bool sing = lu_levels1<kThreads>(G, lu_rec(1), tid, fac, ys, Lv, Uv);
                             sing |= tail_lu(&a.topo[t_id], fac, (int)((unsigned char *)ys - smem),
                                             (int)(ism + L.tail - smem));
                             if (sing) { s_status = GBPF_E_SINGULAR; s_done = 1; }
                             __syncthreads();
-                            for (int l = 0; l < T.t_nbl; l++) {
-                                back_rows<TJ, kThreads>(H, l, grp[3 * l + 2], tid, dinv, Uv, ys);
-                                __syncthreads();
-                            }
+                            back_levels<TJ, kThreads>(G, back_rec(1), tid, dinv, Uv, ys);
                             Ub = nullptr;  // x is there
                         }
                     }
-                    for (int l = 0; !tailed && l < T.nfl; l++) {
+                    if constexpr (kTails) {
+                        if (recs && !tailed && lu_levels1<kThreads>(G, lu_rec(0), tid, fac, ys, Lv, Uv)) {
+                            s_status = GBPF_E_SINGULAR;
+                            s_done = 1;
+                        }
+                        if (recs) __syncthreads();
+                    }
+                    for (int l = 0; !tailed && !recs && l < T.nfl; l++) {
                         if (a.narrow && (G.lvl_narrow[l] & 1)) {
                             if (warp == 0) {
                                 const int gp = a.no_group ? 0 : G.lvl_group_w[3 * l];
@@ -1650,7 +1789,11 @@ __global__ void __launch_bounds__(kThreads, GS == 3 ? 4 : 2) k_nr_block(Args a) 
                 }
                 if (s_done) break;
                 // backward substitution, level by level, narrow levels on warp 0
-                for (int l = 0; Ub && l < T.nbl; l++) {
+                const bool piped = sizeof(TJ) == 4 && T.r_nb[0] && !a.narrow && !a.no_group;
+                if constexpr (sizeof(TJ) == 4) {
+                    if (Ub && piped) back_levels<TJ, kThreads>(G, back_rec(0), tid, Db, Ub, ys);
+                }
+                for (int l = 0; Ub && !piped && l < T.nbl; l++) {
                     if (a.narrow && (G.lvl_narrow[l] & 2)) {
                         if (warp == 0) {
                             back_rows<TJ, 32>(G, l, a.no_group ? 0 : G.lvl_group_w[3 * l + 2], lane, Db, Ub, ys);
@@ -2511,7 +2654,7 @@ struct gbpf_batch {
         const bool fp32 = precision == GBPF_PREC_FP32_IR;
         const Layout w = fp32 ? layout<float>(T.nB, T.n, T.nup, T.nPV, 1, plan.warp_lu1)
                               : layout<double>(T.nB, T.n, T.nup, T.nPV, 1, plan.warp_lu1);
-        return w.total <= (fp32 ? 40u : 56u) * 1024;
+        return w.total <= (fp32 ? kWarpSlice32 : 56u * 1024);
     }
     // learned warm start (solve_warm): features, prediction, chosen start, queue order
     DevBuf warm_mem;
@@ -2681,14 +2824,83 @@ gbpf_status gbpf_batch::add_topology(const Grid &g) {
     o.lvl_rot4 = put(rot4.data(), rot4.size() * 4);
     o.lvl_group4w = put(grp4w.data(), grp4w.size() * 4);
     o.lvl_q4w = put(q4w.data(), q4w.size() * 4);
+    // the records of one set of levels: forward steps and entries, backward rows
+    int r_n[2] = {0, 0}, r_nb[2] = {0, 0};
+    auto records = [&](int v, int nf, const std::vector<int> &fp, const std::vector<int> &fs, const std::vector<int> &ep,
+                       const std::vector<int> &es, const std::vector<int> &lg, const std::vector<int> &rot, int nb,
+                       const std::vector<int> &bp, const std::vector<int> &bs) {
+        auto rounds_of = [](int cnt, int g) { return std::max((cnt + (kThreads >> g) - 1) / (kThreads >> g), 1); };
+        std::vector<int> meta, bmeta;
+        for (int l = 0; l < nf; l++) {
+            const int gp = lg[3 * l], ge = lg[3 * l + 1];
+            const int rounds = std::max(rounds_of(fp[l + 1] - fp[l], gp), rounds_of(ep[l + 1] - ep[l], ge));
+            for (int r = 0; r < rounds; r++) meta.push_back(gp | ge << 3 | (r + 1 == rounds) << 6);
+        }
+        for (int l = 0; l < nb; l++) {
+            const int rounds = rounds_of(bp[l + 1] - bp[l], lg[3 * l + 2]);
+            for (int r = 0; r < rounds; r++) bmeta.push_back(lg[3 * l + 2] | (r + 1 == rounds) << 6);
+        }
+        struct I4 { int x = -1, y = 0, z = 0, w = 0; };
+        struct I2 { int x = 0, y = 0; };
+        std::vector<I4> piv(meta.size() * kThreads), ent(piv.size()), row(bmeta.size() * kThreads);
+        std::vector<I2> ent2(piv.size());
+        std::vector<int> pk(piv.size(), 0);
+        size_t at = 0;
+        for (int l = 0; l < nf; l++) {
+            const int cp = fp[l + 1] - fp[l], ce = ep[l + 1] - ep[l], gp = lg[3 * l], ge = lg[3 * l + 1], rt = rot[l] & 0xffff;
+            for (int w = 0; w < cp; w++)
+                for (int i = 0; i < 1 << gp; i++) {
+                    const int j = fs[fp[l] + w], q = S.dg_ptr[j] + i, qe = S.dg_ptr[j + 1];
+                    const size_t a = at + (w << gp) + i;
+                    piv[a].x = j;
+                    if (q >= qe) continue;
+                    piv[a].y = q; piv[a].z = qe; piv[a].w = S.dg_pos[q];
+                    pk[a] = S.dg_k[q];
+                }
+            // (lane te of the entries is thread te - rot)
+            for (int e = 0; e < ce; e++)
+                for (int i = 0; i < 1 << ge; i++) {
+                    const int p = es[ep[l] + e], q = (int)S.og_ptr[p] + i, qe = (int)S.og_ptr[p + 1];
+                    const size_t te = ((size_t)e << ge) + i;
+                    const size_t a = at + te / kThreads * kThreads + ((te % kThreads + kThreads - rt) & (kThreads - 1));
+                    ent[a].x = p;
+                    if (q >= qe) continue;
+                    ent[a].y = q; ent[a].z = qe; ent[a].w = S.og_a[q];
+                    ent2[a].x = S.og_b[q]; ent2[a].y = S.og_k[q];
+                }
+            at += (size_t)kThreads * std::max(rounds_of(cp, gp), rounds_of(ce, ge));
+        }
+        at = 0;
+        for (int l = 0; l < nb; l++) {
+            const int cnt = bp[l + 1] - bp[l], g = lg[3 * l + 2];
+            for (int w = 0; w < cnt; w++)
+                for (int i = 0; i < 1 << g; i++) {
+                    const int j = bs[bp[l] + w], p = S.up_ptr[j] + i, pe = S.up_ptr[j + 1];
+                    I4 &x = row[at + (w << g) + i];
+                    x.x = j;
+                    if (p >= pe) continue;
+                    x.y = p; x.z = pe; x.w = S.up_col[p];
+                }
+            at += (size_t)kThreads * rounds_of(cnt, g);
+        }
+        auto putv = [&](const auto &x) { return put(x.data(), x.size() * sizeof(x[0])); };
+        o.r_piv[v] = putv(piv); o.r_pk[v] = putv(pk); o.r_ent[v] = putv(ent); o.r_ent2[v] = putv(ent2);
+        o.r_meta[v] = putv(meta); o.r_row[v] = putv(row); o.r_bmeta[v] = putv(bmeta);
+        r_n[v] = (int)meta.size();
+        r_nb[v] = (int)bmeta.size();
+    };
     // the tail form (tail_lu): the dense trailing block of the factor, at most
     // kTailMaxBatch steps; levels of the steps before it and their lanes, and
     // which of their rows each eight threads take into it.  Behind the arrays
     // that a block may stage: it is read where it lies.
     const size_t blob_staged = blob.size();
-    int td = n, t_nfl = 0, t_nbl = 0, t_nsc = 0;
-    if (precision == GBPF_PREC_FP32_IR)
+    int td = n, t_nsc = 0;
+    // (not for grids that run on warps: on blocks, by plan or handed off, those
+    // keep the lists)
+    if (precision == GBPF_PREC_FP32_IR && layout<float>(nB, n, nup, g.nPV, 1, 0).total > kWarpSlice32) {
+        records(0, nfl, S.flev_ptr, S.flev_steps, S.fent_ptr, S.fent_p, grp, rot, nbl, S.blev_ptr, S.blev_steps);
         while (td > 0 && n - td < kTailMaxBatch && S.up_ptr[td] - S.up_ptr[td - 1] == n - td) td--;
+    }
     if (n - td < gbpf::kTailMin) td = n;
     if (td < n) {
         std::vector<std::vector<int>> fl, bl;
@@ -2708,8 +2920,7 @@ gbpf_status gbpf_batch::add_topology(const Grid &g) {
                 if (S.up_col[p] < td) l = std::max(l, lv[S.up_col[p]] + 1);
             add(bl, lv[j] = l, j);
         }
-        t_nfl = (int)fl.size();
-        t_nbl = (int)bl.size();
+        const int t_nfl = (int)fl.size(), t_nbl = (int)bl.size();
         std::vector<int> fp(1, 0), fs, ep(1, 0), es, bp(1, 0), bs, tg(3 * (size_t)std::max(t_nfl, t_nbl), 0), tr(t_nfl + 1, 0);
         for (int l = 0; l < t_nfl; l++) {
             int md = 0, mo = 0;
@@ -2783,8 +2994,7 @@ gbpf_status gbpf_batch::add_topology(const Grid &g) {
             tp.push_back((int)tasks.size());
         }
         auto putv = [&](const std::vector<int> &v) { return put(v.data(), v.size() * 4); };
-        o.t_flev_ptr = putv(fp); o.t_flev_steps = putv(fs); o.t_fent_ptr = putv(ep); o.t_fent_p = putv(es);
-        o.t_blev_ptr = putv(bp); o.t_blev_steps = putv(bs); o.t_group = putv(tg); o.t_rot = putv(tr);
+        records(1, t_nfl, fp, fs, ep, es, tg, tr, t_nbl, bp, bs);
         o.t_dg_end = putv(de); o.t_sc_p = putv(sp); o.t_sc_k = putv(sk); o.t_task_ptr = putv(tp);
         o.t_task = put(tasks.data(), tasks.size() * sizeof(Task));
     }
@@ -2825,7 +3035,11 @@ gbpf_status gbpf_batch::add_topology(const Grid &g) {
     Topo t{};
     t.nB = nB; t.nL = nL; t.n = n; t.nup = nup; t.nnzY = y.nnz; t.nPV = g.nPV; t.nfl = nfl; t.nbl = nbl;
     t.blob_bytes = (int)blob_staged;
-    t.dense = n - td; t.t_nfl = t_nfl; t.t_nbl = t_nbl; t.t_nsc = t_nsc;
+    t.dense = n - td; t.t_nsc = t_nsc;
+    for (int v = 0; v < 2; v++) {
+        t.r_n[v] = r_n[v];
+        t.r_nb[v] = r_nb[v];
+    }
     t.blob = (const char *)mem.p;
     t.o = o;
     grids.push_back(g);

@@ -516,17 +516,23 @@ def test_fp32_bench_scenarios_against_fp64(gb, workload, n):
 # The FP32 step before max|g| <= 1e-8 is below 1e-4 and its relative error eps32 kappa <= 6e-3 (kappa <= 1e5): both
 # forms end within 1e-6 of the FP64 answer, and one more step at most makes up for the rounding.
 @pytest.mark.parametrize("n", [3, 310])
-@pytest.mark.parametrize("nbus,dense", [(83, 15), (87, 16), (107, 16), (20, 19), (240, 38), (400, 67), (470, 78),
-                                        (490, 80), (600, 80)])
+@pytest.mark.parametrize("nbus,dense", [(87, 16), (20, 19), (300, 15), (300, 16), (300, 17), (72, 71), (240, 38), (400, 67),
+                                        (470, 78), (490, 80), (600, 80)])
 def test_batch_fp32_dense_tail(gb, nbus, dense, n):
-    """FP32 thread-block instances of grids that end in a dense trailing block (tail_lu): just under and at its least
-    order, a grid that is all tail, in between, and just over and well over its largest, with shared memory for one
-    block and for two per SM, against the FP64 batch and against the level form (plan narrow)."""
-    if nbus == 20:  # every bus tied to every other
-        f, t = zip(*[(i, j) for i in range(1, 21) for j in range(i + 1, 21)])
-        grid = gb.create_grid(bus_type=[3] + [0] * 19, V0=[1.0] * 20, theta0=[0.0] * 20, from_bus=f, to_bus=t,
-                              r=[0.02] * 190, x=[0.2 + 0.001 * k for k in range(190)],
-                              Pload=[0.0] + [0.1 + 0.02 * k for k in range(19)], Qload=[0.0] + [0.05] * 19)
+    """FP32 thread-block instances of grids that end in a dense trailing block (tail_lu): grids that would run on
+    warps and keep their levels, chains of 300 buses into cliques just under and at its least order, a grid that is all
+    tail, in between, and just over and well over its largest, with shared memory for one block and for two per SM,
+    against the FP64 batch and against the level form (plan narrow)."""
+    if nbus in (20, 72, 300):
+        first = nbus - dense  # the buses before the clique: the slack, or a chain from it
+        br = [(i, i + 1) for i in range(1, first + 1)] if first > 1 else []
+        br += [(i, j) for i in range(first + (first > 1), nbus + 1) for j in range(i + 1, nbus + 1)]
+        f, t = zip(*br)
+        one = nbus / 300 if first > 1 else 1.0
+        grid = gb.create_grid(bus_type=[3] + [0] * (nbus - 1), V0=[1.0] * nbus, theta0=[0.0] * nbus, from_bus=f, to_bus=t,
+                              r=[0.0002 if b <= first else 0.02 for a, b in br],
+                              x=[0.002 * one if b <= first else 0.2 + 0.0001 * b for a, b in br],
+                              Pload=[0.0] + [0.001 + 0.00001 * k for k in range(nbus - 1)], Qload=[0.0] + [0.0005] * (nbus - 1))
     else:
         grid = gb.generate(4, 11, nbus=nbus)
     base = grid.buses()

@@ -577,3 +577,26 @@ def test_batch_spread_over_the_sms_is_exact(gb, prec):
             got = r[k].reshape(n, -1)
             np.testing.assert_array_equal(got, np.asarray(ref[k]).reshape(counts[-1], -1)[:n], err_msg=k)
     assert used[::-1] == [1, 1, 2, 8, 8]
+
+
+@pytest.mark.parametrize("nbus", [3, 14, 31, 34, 60, 97, 118])
+def test_batch_fp32_warp_records(gb, nbus):
+    """FP32 instances on warps, their levels from records of 32 lanes (levels of a lane or two, just under and over a
+    warp's width, several rounds), against the FP64 batch: one more step at most and 1e-6, as for the dense tails."""
+    grid = gb.create_grid(bus_type=[3, 0, 0], V0=[1.0] * 3, theta0=[0.0] * 3, from_bus=[1, 2, 1], to_bus=[2, 3, 3],
+                          r=[0.02] * 3, x=[0.2, 0.25, 0.3], Pload=[0.0, 0.1, 0.2], Qload=[0.0, 0.05, 0.1]) \
+        if nbus == 3 else gb.generate(4, 7, nbus=nbus)
+    base, n = grid.buses(), 40
+    lf = np.random.default_rng(nbus).uniform(0.9, 1.1, (n, grid.nB))
+    Pl, Ql, Pg = base["Pload"] * lf, base["Qload"] * lf, np.tile(base["Pg"], (n, 1))
+    out = []
+    for prec in (gb.PREC_FP64, gb.PREC_FP32_IR):
+        b = gb.Batch([grid], precision=prec, tolerancia=1e-8, no_max_iter=30, lim_inj_reat=0)
+        b.set_instances(np.zeros(n, np.int32), Pload=Pl.ravel(), Qload=Ql.ravel(), Pg=Pg.ravel())
+        b.solve()
+        assert b.plan()["warp_instances"] == n
+        out.append(b.results())
+    ref, r = out
+    assert (r["status"] == 0).all() and (r["iterations"] <= ref["iterations"] + 1).all()
+    for k in ("V", "theta"):
+        np.testing.assert_allclose(r[k], ref[k], rtol=0, atol=1e-6, err_msg=k)

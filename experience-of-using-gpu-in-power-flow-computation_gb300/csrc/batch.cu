@@ -137,6 +137,7 @@ struct TopoOff {
     // of them [0], and of those before the tail [1]
     int r_piv[2], r_pk[2], r_ent[2], r_ent2[2], r_meta[2], r_row[2], r_bmeta[2];
     int r_wlu, r_wback;  // records of the warps' levels (lu_warp_recs)
+    int fent1_ptr, fent1_p;  // the entries of each level that gather anything
 };
 struct Topo {
     int nB, nL, n, nup, nnzY, nPV, nfl, nbl, fac_smem, blob_smem, blob_bytes;
@@ -157,7 +158,7 @@ struct TopoView {
     const int *type, *pv_bus;
     const double *Qmin, *Qmax;
     const int *bus_of_blk, *up_ptr, *up_col, *dg_ptr, *dg_pos, *dg_k, *og_ptr, *og_a, *og_b;
-    const int *flev_ptr, *flev_steps, *blev_ptr, *blev_steps, *ysl, *rbus, *cbus, *fent_ptr, *fent_p, *fent_j;
+    const int *flev_ptr, *flev_steps, *blev_ptr, *blev_steps, *ysl, *rbus, *cbus, *fent_ptr, *fent_p, *fent_j, *fent1_ptr, *fent1_p;
     // log2 of the lanes that share one pivot / one entry / one back-substitution
     // row in the block kernel: [3 * l] pivots and [3 * l + 1] entries of
     // forward level l, [3 * l + 2] rows of backward level l
@@ -200,6 +201,7 @@ __device__ __forceinline__ TopoView bind(const TopoOff &o, const char *b) {
     v.blev_ptr = (const int *)(b + o.blev_ptr); v.blev_steps = (const int *)(b + o.blev_steps);
     v.ysl = (const int *)(b + o.ysl); v.rbus = (const int *)(b + o.rbus); v.cbus = (const int *)(b + o.cbus);
     v.fent_ptr = (const int *)(b + o.fent_ptr); v.fent_p = (const int *)(b + o.fent_p);
+    v.fent1_ptr = (const int *)(b + o.fent1_ptr); v.fent1_p = (const int *)(b + o.fent1_p);
     v.fent_j = (const int *)(b + o.fent_j);
     v.lvl_group = (const int *)(b + o.lvl_group);
     v.lvl_group_w = (const int *)(b + o.lvl_group_w);
@@ -806,7 +808,8 @@ __device__ __forceinline__ void fwd_rows(const TopoView &G, int l, int lg, int t
 //   y_j    = b_j    - sum_k Lt(j,k) z_k,   z_k = D_k^-1 y_k
 //   Lt(i,j) = A_ij  - sum_k Lt(i,k) D_k^-1 U(k,j)
 //   U(j,i)  = A_ji  - sum_k Lt(j,k) D_k^-1 U(k,i)
-// (every k of a gather lies on an earlier level).  The backward
+// (every k of a gather lies on an earlier level; entries without one, half of
+// a tied grid's, stay as the Jacobian fill left them).  The backward
 // substitution is unchanged.  Entries run on lanes rotated by `rot` (a
 // multiple of their group size) so that they overlap the pivots' lanes as
 // little as possible.  Returns true when a pivot block is singular.
@@ -863,12 +866,12 @@ __device__ __forceinline__ bool lu_level1(const TopoView &G, int l, int lgp, int
     {
         const int te = (t + rot) & (NT - 1);
         const int gs = 1 << lge, gl = te & (gs - 1), ng = NT >> lge;
-        const int beg = G.fent_ptr[l], cnt = G.fent_ptr[l + 1] - beg;
+        const int beg = G.fent1_ptr[l], cnt = G.fent1_ptr[l + 1] - beg;
         for (int b0 = 0; b0 < cnt; b0 += ng) {
             const int e = b0 + (te >> lge);
             if (sizeof(TJ) == 8 && b0 + ((te & ~31) >> lge) >= cnt) break;  // none of this warp's
             const bool on = e < cnt;
-            const int p = on ? G.fent_p[beg + e] : 0;
+            const int p = on ? G.fent1_p[beg + e] : 0;
             B4 aL, aU;
             aL.x = aL.y = aL.z = aL.w = (TJ)0;
             aU = aL;
@@ -1025,7 +1028,9 @@ __device__ __forceinline__ bool lu_warp_recs(const TopoView &G, const int4 *rec,
             }
         } else {
             float4 aL = make_float4(0.f, 0.f, 0.f, 0.f), aU = aL;
-            if (lead) { aL = Lv[id]; aU = Uv[id]; }
+            const bool any = q < end;  // (of the lead: without a gather U stays)
+            if (lead) aL = Lv[id];
+            if (lead && any) aU = Uv[id];
             while (q < end) {
                 aL = bms(aL, Lv[y], Uv[x]);
                 aU = bms(aU, Lv[x], Uv[y]);
@@ -1039,7 +1044,7 @@ __device__ __forceinline__ bool lu_warp_recs(const TopoView &G, const int4 *rec,
                 aU = bsum_xor(aU, o);
             }
             if (lead) {
-                Uv[id] = aU;
+                if (any) Uv[id] = aU;
                 Lv[id] = bm(aL, fac[(unsigned)c.z >> 16]);
             }
         }
@@ -1149,12 +1154,12 @@ __device__ __forceinline__ bool lu_level1_q(const TopoView &G, int l, int lgp, i
         // rot is a multiple of 32, so a thread keeps its lane (and quad)
         const int te = (t + rot) & (NT - 1);
         const int tl = te >> 2, gs = 1 << lge, gl = tl & (gs - 1), ng = (NT >> 2) >> lge;
-        const int beg = G.fent_ptr[l], cnt = G.fent_ptr[l + 1] - beg;
+        const int beg = G.fent1_ptr[l], cnt = G.fent1_ptr[l + 1] - beg;
         for (int b0 = 0; b0 < cnt; b0 += ng) {
             const int e = b0 + (tl >> lge);
             if (b0 + ((tl & ~7) >> lge) >= cnt) break;  // none of this warp's
             const bool on = e < cnt;
-            const int p = on ? G.fent_p[beg + e] : 0;
+            const int p = on ? G.fent1_p[beg + e] : 0;
             double aL = 0.0, aU = 0.0;
             if (on && gl == 0) { aL = comp(&Lv[p]); aU = comp(&Uv[p]); }
             if (on)
@@ -1786,7 +1791,14 @@ __global__ void __launch_bounds__(kThreads, GS == 3 ? 4 : 2) k_nr_block(Args a) 
                     Db = facS;
                 } else {
                     // Jacobian fill at every factor position (zeros at fill-in)
-                    for (int q = tid; q < nq; q += kThreads) fac[q] = jac_block<TJ>(G, q, n, act, P, Q, V, cs, sn, f32);
+                    // (two blocks at a time: their loads go out together)
+                    for (int q = tid; q < nq; q += 2 * kThreads) {
+                        const int q1 = min(q + kThreads, nq - 1);
+                        const B4 b0 = jac_block<TJ>(G, q, n, act, P, Q, V, cs, sn, f32);
+                        const B4 b1 = jac_block<TJ>(G, q1, n, act, P, Q, V, cs, sn, f32);
+                        fac[q] = b0;
+                        if (q + kThreads < nq) fac[q1] = b1;
+                    }
                     __syncthreads();
                     // LU factorisation fused with forward substitution, one level at a
                     // time, in two passes: pivots (diagonal block, its inverse, y_j),
@@ -2819,6 +2831,13 @@ gbpf_status gbpf_batch::add_topology(const Grid &g) {
     o.blev_ptr = put(S.blev_ptr.data(), (nbl + 1) * 4); o.blev_steps = put(S.blev_steps.data(), n * 4);
     o.ysl = put(S.ysl.data(), nq * 4); o.rbus = put(S.rbus.data(), nq * 4); o.cbus = put(S.cbus.data(), nq * 4);
     o.fent_ptr = put(S.fent_ptr.data(), (nfl + 1) * 4); o.fent_p = put(S.fent_p.data(), nup * 4);
+    std::vector<int> f1_ptr(1, 0), f1_p;
+    for (int l = 0; l < nfl; l++) {
+        for (int e = S.fent_ptr[l]; e < S.fent_ptr[l + 1]; e++)
+            if (S.og_ptr[S.fent_p[e]] < S.og_ptr[S.fent_p[e] + 1]) f1_p.push_back(S.fent_p[e]);
+        f1_ptr.push_back((int)f1_p.size());
+    }
+    o.fent1_ptr = put(f1_ptr.data(), f1_ptr.size() * 4); o.fent1_p = put(f1_p.data(), f1_p.size() * 4);
     o.fent_j = put(S.fent_j.data(), nup * 4);
     // lanes per pivot / entry / row of each level for the block kernel: as many
     // as the level's thread budget allows, no more than its longest list needs
@@ -3052,7 +3071,7 @@ gbpf_status gbpf_batch::add_topology(const Grid &g) {
     // (not for grids that run on warps: on blocks, by plan or handed off, those
     // keep the lists)
     if (precision == GBPF_PREC_FP32_IR && !on_warps) {
-        records(0, nfl, S.flev_ptr, S.flev_steps, S.fent_ptr, S.fent_p, grp, rot, nbl, S.blev_ptr, S.blev_steps);
+        records(0, nfl, S.flev_ptr, S.flev_steps, f1_ptr, f1_p, grp, rot, nbl, S.blev_ptr, S.blev_steps);
         while (td > 0 && n - td < kTailMaxBatch && S.up_ptr[td] - S.up_ptr[td - 1] == n - td) td--;
     }
     if (n - td < gbpf::kTailMin) td = n;
@@ -3082,7 +3101,7 @@ gbpf_status gbpf_batch::add_topology(const Grid &g) {
                 fs.push_back(j);
                 md = std::max(md, S.dg_ptr[j + 1] - S.dg_ptr[j]);
                 for (int p = S.up_ptr[j]; p < S.up_ptr[j + 1]; p++) {
-                    es.push_back(p);
+                    if (S.og_ptr[p] < S.og_ptr[p + 1]) es.push_back(p);
                     mo = std::max(mo, (int)(S.og_ptr[p + 1] - S.og_ptr[p]));
                 }
             }

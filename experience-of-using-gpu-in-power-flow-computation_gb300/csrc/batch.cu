@@ -2789,7 +2789,6 @@ struct gbpf_batch {
     } plan;
     int block_gs = 0;  // placement level of the block-mode launch's state (layout gs)
     int warp_gs = 0;   // ... and of the warp launch's
-    int block_carve = -1, warp_carve = -1;  // division of L1 and shared memory that they ask for
     DevBuf gstate_mem, warp_gstate_mem;
     gbpf_status rebuild() {
         CK(cudaStreamSynchronize(stream));
@@ -3340,21 +3339,9 @@ gbpf_status gbpf_batch::set_instances(int n, const int *tofi, const double *Ploa
 
 gbpf_status gbpf_batch::launch(cudaStream_t st) { return launch_with(st, args, wargs, true); }
 
-// carve: share of the SM's L1 and shared memory, in percent, that the launch
-// asks for as shared memory (-1: the driver's choice)
-static void launch_kernel(const void *fn, int grid, int threads, size_t smem, cudaStream_t st, const Args &a, int carve) {
-    cudaLaunchConfig_t c{};
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-    at.val.sharedMemCarveout = (unsigned)carve;
-    c.gridDim = dim3(grid);
-    c.blockDim = dim3(threads);
-    c.dynamicSmemBytes = smem;
-    c.stream = st;
-    c.attrs = &at;
-    c.numAttrs = carve >= 0;
+static void launch_kernel(const void *fn, int grid, int threads, size_t smem, cudaStream_t st, const Args &a) {
     void *args[] = {(void *)&a};
-    cudaLaunchKernelExC(&c, fn, args);
+    (void)cudaLaunchKernel(fn, dim3(grid), dim3(threads), args, smem, st);
 }
 
 // One persistent launch per mode over the queues of ba (blocks) and wa (warps).
@@ -3366,7 +3353,7 @@ gbpf_status gbpf_batch::launch_with(cudaStream_t st, const Args &ba, const Args 
         CK(cudaStreamWaitEvent(side, fork, 0));
         if (timed) CK(cudaEventRecordWithFlags(kev[0], side, cudaEventRecordExternal));
         launch_kernel(fp32 ? blk_kernel<float>(block_gs) : blk_kernel<double>(block_gs), grid_blocks, kThreads, smem, side,
-                      ba, block_carve);
+                      ba);
         {
             const cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) {
@@ -3385,7 +3372,7 @@ gbpf_status gbpf_batch::launch_with(cudaStream_t st, const Args &ba, const Args 
     if (wa.queue_len) {
         if (timed) CK(cudaEventRecordWithFlags(kev[2], st, cudaEventRecordExternal));
         launch_kernel(fp32 ? warp_kernel<float>(warp_gs) : warp_kernel<double>(warp_gs), warp_grid, 32 * warp_warps,
-                      warp_smem, st, wa, warp_carve);
+                      warp_smem, st, wa);
         CK_LAUNCH();
         if (timed) CK(cudaEventRecordWithFlags(kev[3], st, cudaEventRecordExternal));
         if (wa.handoff_it > 0) {
@@ -3447,32 +3434,20 @@ gbpf_status gbpf_batch::build_graph() {
     CK(cudaMalloc(&queues.p, 4 * (size_t)n_inst + 256));
     if (n_warp_q) CK(cudaMemcpy(queues.p, wq.data(), 4 * wq.size(), cudaMemcpyHostToDevice));
     if (n_block_q) CK(cudaMemcpy((int *)queues.p + n_warp_q, bq.data(), 4 * bq.size(), cudaMemcpyHostToDevice));
-    // Where one kernel has the SMs to itself, it asks for the shared memory of
-    // its blocks and no more: the rest is L1, where the index lists and global
-    // factors are read from; left alone, the driver makes room for as many
-    // blocks as would fit (2,048 FP32 instances of a 1,888-bus grid 6.78 ->
-    // 6.60 ms, 57 buses at one warp to a block 0.20 -> 0.165).  When both run,
-    // the choice stays the driver's: an SM takes a block only when its division
-    // suits.
-    int sm_smem = 0;
-    CK(cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
-    auto carve_of = [&](int blocks, size_t dyn) {  // blocks of dyn bytes and static and reserved ones
-        const size_t want = 100 * (size_t)blocks * (dyn + 1280);
-        return (int)std::min<size_t>(100, (want + sm_smem - 1) / sm_smem);
-    };
-    block_carve = warp_carve = -1;
     // Block-mode shared-memory plan: the blob is staged in shared memory when
     // at most 48 KB; the factor stays in shared memory when blob region +
     // state + factor fit in 110 KB, otherwise it lives in global scratch.
     // With plan.gstate the plan is also made with part of the state in global
     // memory (layout gs), and that one is taken when it fits more blocks per
-    // SM that have work, or as many with more factors and tails in shared
-    // memory.  A tail has its place before the factor.  With an instance per SM
-    // or fewer the factor may take the whole of shared memory (150 FP32
-    // instances of a 1,888-bus grid: 1.03 -> 0.91 ms).
-    const int per_sm = (n_block_q + dev_sm - 1) / dev_sm;  // blocks that there is work for
-    const size_t budget = per_sm <= 1 && !n_warp_q && plan.gstate == 1 ? (size_t)maxsm - 1024 : 110 * 1024;
-    const size_t blob_cap = 48 * 1024;
+    // SM, or as many with more factors and tails in shared memory.  A tail has
+    // its place before the factor.  The plan looks at the grids alone and not
+    // at the number of instances: other batches may be in flight beside this
+    // one, on their own streams, and a plan (or a division of L1 and shared
+    // memory asked for at the launch) that gives a small batch all of an SM
+    // makes them wait for one another.  Four batches of 100 FP32 instances of a
+    // 1,888-bus grid launched together: 1.78 ms with the whole SM planned for
+    // one, 1.07 as it is (alone 0.55 and 0.71).
+    const size_t budget = 110 * 1024, blob_cap = 48 * 1024;
     size_t region = 0;
     for (size_t t = 0; t < topo_h.size(); t++) {
         Topo &T = topo_h[t];
@@ -3531,7 +3506,6 @@ gbpf_status gbpf_batch::build_graph() {
         if (!n_block_q || sm > (size_t)maxsm) return GBPF_OK;
         CK(cudaFuncSetAttribute(blk_fn(gs), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bp.occ, blk_fn(gs), kThreads, sm));
-        bp.occ = std::min(bp.occ, per_sm);
         return GBPF_OK;
     };
     // Placement level: gstate 2 / 3 / 4 take level 1 / 2 / 3 where it fits;
@@ -3619,7 +3593,6 @@ gbpf_status gbpf_batch::build_graph() {
     gstate_mem.reset();
     args.gstate = nullptr;
     args.gstate_stride = block_gs ? (long long)align_up(bp.gst, 256) : 0;
-    if (n_block_q && !n_warp_q) block_carve = carve_of((grid_blocks + dev_sm - 1) / dev_sm, smem);
     if (block_gs) {
         CK(cudaMalloc(&gstate_mem.p, (size_t)args.gstate_stride * grid_blocks));
         args.gstate = (unsigned char *)gstate_mem.p;
@@ -3682,7 +3655,6 @@ gbpf_status gbpf_batch::build_graph() {
         warp_warps = wp.warps;
         warp_smem = (size_t)warp_warps * slice;
         warp_grid = std::max(1, std::min((n_warp_q + warp_warps - 1) / warp_warps, dev_sm * std::max(wp.occ, 1)));
-        if (!n_block_q) warp_carve = carve_of((warp_grid + dev_sm - 1) / dev_sm, warp_smem);
         warp_gstride = warp_gs ? align_up(wp.gst, 256) : 0;
     }
     warp_gstate_mem.reset();

@@ -2666,6 +2666,18 @@ __global__ void k_pack_inputs(PackArgs a) {
 // ---------------------------------------------------------------------------
 // host object
 // ---------------------------------------------------------------------------
+// Lets launches of a kernel ask for as much dynamic shared memory as a block
+// can have.  The limit is one value for all launches of a kernel on a device:
+// set to what one batch needs, it would refuse the launches of a larger batch
+// that was built before, so it is the same whoever sets it.
+gbpf_status opt_in_smem(const void *fn, int device) {
+    int optin = 0;
+    cudaFuncAttributes fa{};
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    CK(cudaFuncGetAttributes(&fa, fn));
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+    return GBPF_OK;
+}
 // The block kernel of a state placement level (layout gs), as a function
 // handle for attributes and occupancy queries.
 template <typename TJ> const void *warp_kernel(int gs) {
@@ -3504,7 +3516,7 @@ gbpf_status gbpf_batch::build_graph() {
         }
         const size_t sm = bp.need + region;
         if (!n_block_q || sm > (size_t)maxsm) return GBPF_OK;
-        CK(cudaFuncSetAttribute(blk_fn(gs), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        if (const gbpf_status st = opt_in_smem(blk_fn(gs), device)) return st;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bp.occ, blk_fn(gs), kThreads, sm));
         return GBPF_OK;
     };
@@ -3573,13 +3585,9 @@ gbpf_status gbpf_batch::build_graph() {
     const bool use_handoff = n_warp_q > 0 && plan.handoff_it > 0 && max_iter > plan.handoff_it;
     grid_blocks = 0;
     resume_grid = 0;
-    {
-        // the resume launch always keeps its state in shared memory
-        size_t attr_sm = use_handoff ? resume_smem : 0;
-        if (!block_gs) attr_sm = std::max(attr_sm, smem);
-        if (attr_sm) CK(cudaFuncSetAttribute(blk_fn(0), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attr_sm));
-        if (block_gs) CK(cudaFuncSetAttribute(blk_fn(block_gs), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    }
+    // (the resume launch always keeps its state in shared memory)
+    for (int gs : {0, block_gs})
+        if (const gbpf_status st = opt_in_smem(blk_fn(gs), device)) return st;
     if (n_block_q) {
         int occ = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, blk_fn(block_gs), kThreads, smem));
@@ -3631,7 +3639,7 @@ gbpf_status gbpf_batch::build_graph() {
             wp.warps = std::min(wp.warps, per_sm_w);
             const size_t sm = (size_t)wp.warps * wp.slice;
             const void *fn = fp32 ? warp_kernel<float>(gs) : warp_kernel<double>(gs);
-            CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            if (const gbpf_status st = opt_in_smem(fn, device)) return st;
             CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wp.occ, fn, 32 * wp.warps, sm));
             return GBPF_OK;
         };
@@ -3684,10 +3692,10 @@ gbpf_status gbpf_batch::build_graph() {
             // opt-in limit (FP64 past ~13,900 buses) the topology has no shared
             // iteration 0 and its instances compute their own
             if (fs > (size_t)maxsm) continue;
-            if (fs > 48 * 1024) {
-                if (fp32) CK(cudaFuncSetAttribute(k_flat_start<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs));
-                else CK(cudaFuncSetAttribute(k_flat_start<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs));
-            }
+            if (fs > 48 * 1024)
+                if (const gbpf_status st = opt_in_smem(fp32 ? (const void *)k_flat_start<float> : (const void *)k_flat_start<double>,
+                                                       device))
+                    return st;
             if (fp32) k_flat_start<float><<<1, 32, fs, stream>>>(T, o, plan.warp_group, plan.quad);
             else k_flat_start<double><<<1, 32, fs, stream>>>(T, o, plan.warp_group, plan.quad);
             CK_LAUNCH();
@@ -3818,7 +3826,7 @@ gbpf_status gbpf_batch::warm_launch(gbpf_mlp *m) {
         CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
         if (sel <= (size_t)optin) {
             if (sel > 48 * 1024)
-                CK(cudaFuncSetAttribute(k_ws_select<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel));
+                if ((st = opt_in_smem((const void *)k_ws_select<true>, device)) != GBPF_OK) return st;
             k_ws_select<true><<<n_inst, kSelThreads, sel, stream>>>(args, wPred, sh.outp, sh.out_mean, sh.out_scale,
                                                                     wV, wTh, wEF, wKind, wCls, wHist);
         } else {
@@ -3882,10 +3890,10 @@ gbpf_status gbpf_batch::make_wref(const gbpf::MlpShape &sh, int t0) {
         char *o = (char *)wref_mem.p;
         CK(cudaMemcpyAsync(o + F.V0, wref_h.data(), 8 * (size_t)T.nB, cudaMemcpyHostToDevice, stream));
         CK(cudaMemcpyAsync(o + F.th0, wref_h.data() + T.nB, 8 * (size_t)T.nB, cudaMemcpyHostToDevice, stream));
-        if (fs > 48 * 1024) {
-            if (fp32) CK(cudaFuncSetAttribute(k_flat_start<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs));
-            else CK(cudaFuncSetAttribute(k_flat_start<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs));
-        }
+        if (fs > 48 * 1024)
+            if (const gbpf_status st = opt_in_smem(fp32 ? (const void *)k_flat_start<float> : (const void *)k_flat_start<double>,
+                                                   device))
+                return st;
         if (fp32) k_flat_start<float><<<1, 32, fs, stream>>>(T, o, plan.warp_group, plan.quad);
         else k_flat_start<double><<<1, 32, fs, stream>>>(T, o, plan.warp_group, plan.quad);
         CK_LAUNCH();
@@ -4243,7 +4251,7 @@ extern "C" gbpf_status gbpf_batch_solve_noalloc(gbpf_batch *b, int n_inst, const
     else CK(cudaFuncGetAttributes(&fa, k_nr_block<double, 0>));
     if ((size_t)fa.maxDynamicSharedSizeBytes < smem) {
         const void *fn = fp32 ? (const void *)k_nr_block<float, 0> : (const void *)k_nr_block<double, 0>;
-        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (const gbpf_status st = opt_in_smem(fn, b->device)) return st;
     }
     if (fp32) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_nr_block<float, 0>, kThreads, smem));
     else CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_nr_block<double, 0>, kThreads, smem));

@@ -974,12 +974,12 @@ struct gbpf_solver {
     }
     void launch_dense_solve(int guard) {
         cudaLaunchAttribute at[1];
-        cudaLaunchConfig_t cfg = cluster_config(kDCtas, dense_back_smem(), at);
+        cudaLaunchConfig_t cfg = cluster_config(kDCtas, dense_back_smem(d.N), at);
         cfg.blockDim = dim3(kDBackThreads);
         (void)cudaLaunchKernelEx(&cfg, k_dback, d, guard);
     }
-    size_t dense_back_smem() const {
-        return sizeof(double) * 5 * kDPanel * (size_t)cdiv_int(cdiv_int(d.N, kDPanel), kDCtas);
+    static size_t dense_back_smem(int N) {
+        return sizeof(double) * 5 * kDPanel * (size_t)cdiv_int(cdiv_int(N, kDPanel), kDCtas);
     }
     void launch_eval(int guard) {  // injections, limits, mismatch
         const int T = 256;
@@ -1323,7 +1323,8 @@ gbpf_status gbpf_solver::build_graph() {
         CK(cudaFuncSetAttribute(k_dpanel_cl, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kDPanRows * kDPanLd * (int)sizeof(double)));
         CK(cudaFuncSetAttribute(k_dback, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        CK(cudaFuncSetAttribute(k_dback, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dense_back_smem()));
+        // (one limit for all solvers: the largest system's)
+        CK(cudaFuncSetAttribute(k_dback, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dense_back_smem(kDenseMaxN)));
     }
     CK(cudaGraphCreate(&graph, 0));
     cudaGraphConditionalHandle h;

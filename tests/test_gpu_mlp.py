@@ -460,3 +460,36 @@ def test_training_steps_side_by_side_repeat_their_bits(gb, width, layers, n_out,
                 continue
             stable = np.abs(ga) > 1e-2 * np.max(np.abs(ga))  # the first step is lr against the gradient's sign
             assert np.max(np.abs((a1 - a0) + 1e-3 * np.sign(ga))[stable]) < 1e-5
+
+
+@pytest.mark.parametrize("prec", ["PREC_FP64", "PREC_FP32_IR"])
+@pytest.mark.parametrize("name,counts", [("c4_118.cdf.gz", (2048, 100)), ("c4_118.cdf.gz", (100, 2048)),
+                                         ("c5_base.cdf.gz", (100, 400)), ("c5_base.cdf.gz", (400, 100))])
+def test_warm_launch_beside_a_batch_of_another_size(gb, name, counts, prec):
+    """A warm-started launch asks for the shared memory of its own batch, whatever batches of the same grid were built
+    after it: same bits before and after, and the other batch's solve is its own too."""
+    import bench
+
+    grid = gb.read_grid(bench.grid_file(name))
+    base, nB = grid.buses(), grid.nB
+    m = gb.MLP(2 * nB, 2 * nB, width=64, n_layers=1, skip=False, seed=3)
+    m.set_norm(np.zeros(2 * nB), np.ones(2 * nB), np.concatenate([base["V0"], base["theta0"]]), np.full(2 * nB, 1e-3))
+    lf = np.random.default_rng(4).uniform(0.95, 1.05, (max(counts), nB))
+    bs = [gb.Batch([grid], precision=getattr(gb, prec), tolerancia=1e-8, no_max_iter=30, lim_inj_reat=0) for _ in counts]
+
+    def fill(b, n):
+        b.set_instances(np.zeros(n, np.int32), Pload=(base["Pload"] * lf[:n]).ravel(), Qload=(base["Qload"] * lf[:n]).ravel())
+
+    fill(bs[0], counts[0])
+    bs[0].solve_warm(m)
+    before = bs[0].results()
+    assert (before["status"] == 0).all()
+    fill(bs[1], counts[1])
+    bs[0].solve_warm(m)
+    after = bs[0].results()
+    bs[1].solve_warm(m)
+    other = bs[1].results()
+    for k in ("V", "theta", "iterations", "status"):
+        np.testing.assert_array_equal(after[k], before[k], err_msg=k)
+        n = min(counts) * (nB if k in ("V", "theta") else 1)
+        np.testing.assert_array_equal(other[k][:n], before[k][:n], err_msg=k)

@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -2818,7 +2819,8 @@ struct gbpf_batch {
     }
     // learned warm start (solve_warm): features, prediction, chosen start, queue order
     DevBuf warm_mem;
-    int warm_n = 0;
+    // instances, their buses, the network's padded inputs and outputs that warm_mem is laid out for
+    std::array<long long, 4> warm_key{};
     __nv_bfloat16 *wX = nullptr;
     float *wPred = nullptr;
     double *wV = nullptr, *wTh = nullptr;
@@ -3785,7 +3787,9 @@ gbpf_status gbpf_batch::warm_launch(gbpf_mlp *m) {
         return GBPF_E_ARG;
     }
     if (sh.device != device) { set_error("network and batch live on different devices"); return GBPF_E_ARG; }
-    if (warm_n != n_inst) {
+    const std::array<long long, 4> key{n_inst, n_bus_total, sh.kin, sh.outp};
+    if (warm_key != key) {
+        warm_key = {};
         warm_mem.reset();
         if (h_kind) { cudaFreeHost(h_kind); h_kind = nullptr; }
         if (h_witers) { cudaFreeHost(h_witers); h_witers = nullptr; }
@@ -3801,7 +3805,7 @@ gbpf_status gbpf_batch::warm_launch(gbpf_mlp *m) {
         p += 4 * vb;
         wKind = (int *)p; wQueue = (int *)(p + ib); wIters = (int *)(p + 2 * ib); wCls = (int *)(p + 3 * ib);
         wHist = (int *)(p + 4 * ib);  // class counts, then the order's cursors
-        warm_n = n_inst;
+        warm_key = key;
     }
     if (!mwork) mwork = gbpf::mlp_work_create();
     gbpf_status st0;

@@ -493,3 +493,35 @@ def test_warm_launch_beside_a_batch_of_another_size(gb, name, counts, prec):
         np.testing.assert_array_equal(after[k], before[k], err_msg=k)
         n = min(counts) * (nB if k in ("V", "theta") else 1)
         np.testing.assert_array_equal(other[k][:n], before[k][:n], err_msg=k)
+
+
+@pytest.mark.parametrize("prec", ["PREC_FP64", "PREC_FP32_IR"])
+def test_warm_start_on_another_grid_and_another_network(gb, prec):
+    """As many instances as before, but on the batch's other grid, or with a network of other inputs: each warm-started
+    solve has the bits of a batch that never ran another."""
+    import bench
+
+    grids = [gb.read_grid(bench.grid_file(f)) for f in ("c4_14.cdf.gz", "c4_118.cdf.gz")]
+    n = 40
+
+    def net(grid, k):
+        base, nB = grid.buses(), grid.nB
+        m = gb.MLP(k * nB, 2 * nB, width=64, n_layers=1, skip=False, seed=3)
+        m.set_norm(np.zeros(k * nB), np.ones(k * nB), np.concatenate([base["V0"], base["theta0"]]), np.full(2 * nB, 1e-3))
+        return m
+
+    def solve(b, t, m):
+        base = grids[t].buses()
+        lf = np.random.default_rng(t).uniform(0.95, 1.05, (n, grids[t].nB))
+        b.set_instances(np.full(n, t, np.int32), Pload=(base["Pload"] * lf).ravel(), Qload=(base["Qload"] * lf).ravel())
+        w = b.solve_warm(m)
+        return dict(b.results(), kind=w["start_kind"])
+
+    new = lambda: gb.Batch(grids, precision=getattr(gb, prec), tolerancia=1e-8, no_max_iter=30, lim_inj_reat=0)
+    nets = {(t, k): net(grids[t], k) for t in (0, 1) for k in (2, 3)}
+    b = new()
+    for t, k in ((0, 2), (0, 3), (1, 2), (1, 3), (0, 3), (1, 3)):
+        r, ref = solve(b, t, nets[t, k]), solve(new(), t, nets[t, k])
+        assert (r["status"] == 0).all()
+        for key in ("V", "theta", "iterations", "kind"):
+            np.testing.assert_array_equal(r[key], ref[key], err_msg=f"{t} {k} {key}")

@@ -806,7 +806,8 @@ struct gbpf_mlp {
     // CTA (at most one CTA per SM splits) and one arrival counter per tile
     Dev splitk;
     float *ws[3] = {};    // ... for the chain, the side and the hidden weight gradients (Fork)
-    int *ws_cnt[3] = {};
+    int *ws_cnt[3] = {};  // one behind the other, ws_cnt_bytes in all
+    size_t ws_cnt_bytes = 0;
     std::vector<float> in_mean, in_iscale, out_mean, out_scale;  // host copies
     float *d_in_mean = nullptr, *d_in_iscale = nullptr, *d_out_mean = nullptr, *d_out_scale = nullptr;
     int *d_t = nullptr, *d_err = nullptr;
@@ -947,7 +948,8 @@ gbpf_status gbpf_mlp::init(int n_in_, int hidden_, int n_hidden_, int n_out_, in
         const int ncnt = BNmax / kBoxB * sms;
         CK(cudaMalloc(&splitk.p, 3 * (part + 4 * (size_t)ncnt)));
         int *cnt = (int *)((char *)splitk.p + 3 * part);
-        CK(cudaMemset(cnt, 0, 3 * 4 * (size_t)ncnt));
+        ws_cnt_bytes = 3 * 4 * (size_t)ncnt;
+        CK(cudaMemset(cnt, 0, ws_cnt_bytes));
         for (int q = 0; q < 3; q++) {
             ws[q] = (float *)((char *)splitk.p + q * part);
             ws_cnt[q] = cnt + q * ncnt;
@@ -1277,12 +1279,16 @@ gbpf_status mlp_infer(gbpf_mlp *m, const bf16 *X, int n, float *out, cudaStream_
 
 namespace {
 // The network's error word (set by a GEMM whose wait ran out): read after a
-// call's GEMMs and cleared, so that the next call starts clean.
+// call's GEMMs and cleared, so that the next call starts clean.  With it the
+// arrival counts of the split tiles: a split that ran out does not arrive, and
+// a count left in between would let the next call sum partials that are not
+// there yet.
 gbpf_status take_err(gbpf_mlp *m) {
     int err = 0;
     CK(cudaMemcpy(&err, m->d_err, 4, cudaMemcpyDeviceToHost));
     if (!err) return GBPF_OK;
-    CK(cudaMemset(m->d_err, 0, 4));
+    CK(cudaMemsetAsync(m->d_err, 0, 4, m->stream));
+    CK(cudaMemsetAsync(m->ws_cnt[0], 0, m->ws_cnt_bytes, m->stream));
     set_error("a tensor-core GEMM wait ran out");
     return GBPF_E_TIMEOUT;
 }

@@ -525,3 +525,33 @@ def test_warm_start_on_another_grid_and_another_network(gb, prec):
         assert (r["status"] == 0).all()
         for key in ("V", "theta", "iterations", "kind"):
             np.testing.assert_array_equal(r[key], ref[key], err_msg=f"{t} {k} {key}")
+
+
+def test_split_gemms_recover_from_waits_that_ran_out(gb):
+    """GEMMs whose K is split over CTAs count the splits that arrived.  Where the wait limit lets some splits of a tile
+    run out and others arrive (limits from below one TMA load to a few of them), the counts are left in between; the
+    next call with the default limit must not take them over: gradients bit for bit those from before."""
+    rng = np.random.default_rng(31)
+    m = gb.MLP(3072, 64, width=64, n_layers=2, skip=True, seed=31)
+    X, Y = rng.normal(size=(1024, 3072)).astype(np.float32), rng.normal(size=(1024, 64)).astype(np.float32)
+
+    def grads():
+        loss, g = m.gradients(X, Y)
+        return [np.float32(loss)] + [a for l in g for a in l if a is not None]
+
+    before = grads()
+    for a, b in zip(grads()[1:], before[1:]):
+        np.testing.assert_array_equal(a, b)
+    ran_out = 0
+    for limit in (300, 600, 800, 1000, 1200, 1400, 1600, 1800, 2000, 2400, 2800, 3200, 4000, 5000):
+        for _ in range(3):
+            m.set_wait_limit(limit)
+            try:
+                grads()
+            except gb.GbpfError as e:
+                assert e.status == gb.E_TIMEOUT
+                ran_out += 1
+            m.set_wait_limit(0)
+            for a, b in zip(grads()[1:], before[1:]):
+                np.testing.assert_array_equal(a, b, err_msg=str(limit))
+    assert ran_out > 0

@@ -114,10 +114,12 @@ struct EpiArgs {
     int *ws_cnt;
 };
 
-// Learning rate of Adam step t (1-based): cosine decay from lr to sched[2]
-// over the sched[1] steps that start after step sched[0].
-__device__ __forceinline__ float sched_lr(float lr, const float *sched, int t) {
-    const float T = sched[1];
+// Learning rate of Adam step t (1-based): cosine decay from sched[3] to sched[2]
+// over the sched[1] steps that start after step sched[0] (0: constant).  All of
+// it is read from the device: the training graph outlives the call it was
+// captured in.
+__device__ __forceinline__ float sched_lr(const float *sched, int t) {
+    const float T = sched[1], lr = sched[3];
     if (!(T > 0.f)) return lr;
     const float f = fminf(1.f, fmaxf(0.f, ((float)t - sched[0]) / T));
     return sched[2] + 0.5f * (lr - sched[2]) * (1.f + cospif(f));
@@ -501,8 +503,8 @@ struct BiasJobs {
 
 // Bias gradient = column sum of dZ over the batch = row sum of dZ^T; then
 // Adam on the bias (or store the gradient).  One warp per bias entry.
-__global__ void k_bias(BiasJobs J, const int *adam_t, int step, const float *sched, float lr, float b1, float b2,
-                       float eps, int adam) {
+__global__ void k_bias(BiasJobs J, const int *adam_t, int step, const float *sched, float b1, float b2, float eps,
+                       int adam) {
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (gw >= J.row_start[J.njobs]) return;
     int j = 0;
@@ -519,7 +521,7 @@ __global__ void k_bias(BiasJobs J, const int *adam_t, int step, const float *sch
     const float m = b1 * J.bm[j][r] + (1.f - b1) * s, v = b2 * J.bv[j][r] + (1.f - b2) * s * s;
     J.bm[j][r] = m;
     J.bv[j][r] = v;
-    J.b[j][r] -= sched_lr(lr, sched, ti) * (m / (1.f - powf(b1, t))) / (sqrtf(v / (1.f - powf(b2, t))) + eps);
+    J.b[j][r] -= sched_lr(sched, ti) * (m / (1.f - powf(b1, t))) / (sqrtf(v / (1.f - powf(b2, t))) + eps);
 }
 
 // Adam on the weights of several layers in one streaming pass, after the
@@ -541,10 +543,10 @@ struct AdamJobs {
 };
 constexpr int kAdamU = 4;
 
-__global__ void __launch_bounds__(256) k_adam(AdamJobs J, const int *adam_t, int step, const float *sched, float lr,
-                                              float b1, float b2, float eps) {
+__global__ void __launch_bounds__(256) k_adam(AdamJobs J, const int *adam_t, int step, const float *sched, float b1,
+                                              float b2, float eps) {
     const int ti = *adam_t + 1 + step;
-    const float t = (float)ti, lrt = sched_lr(lr, sched, ti);
+    const float t = (float)ti, lrt = sched_lr(sched, ti);
     const float c1 = 1.f / (1.f - powf(b1, t)), c2 = 1.f / (1.f - powf(b2, t));
     const long long total = J.start[J.njobs], stride = (long long)gridDim.x * blockDim.x;
     for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; i0 < total; i0 += stride * kAdamU) {
@@ -836,7 +838,6 @@ struct gbpf_mlp {
     // inference workspace
     Work iw;
     int iw_cap = 0;
-    float lr = 1e-3f;
     float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     // loss metric: loss = (|e A|^2 + lam |e|^2) / (rows * n_out) over the
     // normalised output residual e, A [n_out, k]; without A, plain mean
@@ -958,7 +959,7 @@ gbpf_status gbpf_mlp::init(int n_in_, int hidden_, int n_hidden_, int n_out_, in
     d_t = (int *)misc.p;
     d_err = d_t + 1;
     d_loss = (float *)(d_t + 2);
-    d_sched = (float *)(d_t + 4);  // 3 floats, zero = constant learning rate
+    d_sched = (float *)(d_t + 4);  // 4 floats (sched_lr)
     CK(cudaStreamSynchronize(stream));
     return GBPF_OK;
 }
@@ -1121,7 +1122,7 @@ gbpf_status gbpf_mlp::adam_layers(cudaStream_t st, std::initializer_list<std::pa
         }
     const long long groups = A.start[A.njobs];
     const int blocks = (int)std::max(1LL, (groups + 256 * kAdamU - 1) / (256 * kAdamU));
-    k_adam<<<blocks, 256, 0, st>>>(A, d_t, step, d_sched, lr, b1, b2, eps);
+    k_adam<<<blocks, 256, 0, st>>>(A, d_t, step, d_sched, b1, b2, eps);
     CK(cudaGetLastError());
     return GBPF_OK;
 }
@@ -1212,7 +1213,7 @@ gbpf_status gbpf_mlp::backward(cudaStream_t st, Work &w, const CUtensorMap &mXT,
         J.row_start[l + 1] = J.row_start[l] + L[l].out;
     }
     const int warps = J.row_start[nl];
-    k_bias<<<(warps * 32 + 255) / 256, 256, 0, wg>>>(J, d_t, step, d_sched, lr, b1, b2, eps, adam ? 1 : 0);
+    k_bias<<<(warps * 32 + 255) / 256, 256, 0, wg>>>(J, d_t, step, d_sched, b1, b2, eps, adam ? 1 : 0);
     CK(cudaGetLastError());
     if ((s = order(f ? f->hidden : nullptr, wg, st)) != GBPF_OK) return s;
     if (!adam) return GBPF_OK;
@@ -1372,7 +1373,6 @@ extern "C" gbpf_status gbpf_mlp_train(gbpf_mlp *m, int epochs, int batch, float 
     ARG(m->n_data >= batch);
     CK(cudaSetDevice(m->device));
     const int n = m->n_data, steps = n / batch;
-    m->lr = lr;
     if (!m->exec || m->graph_B != batch) {
         if (m->exec) { cudaGraphExecDestroy(m->exec); m->exec = nullptr; }
         gbpf_status s = m->make_work(m->tw, batch, true);
@@ -1417,7 +1417,7 @@ extern "C" gbpf_status gbpf_mlp_train(gbpf_mlp *m, int epochs, int batch, float 
     }
     // the schedule of this call: cosine from lr to lr_final over its steps
     // (lr_final == lr: constant), read by the Adam kernels from the device
-    const float sched[3] = {(float)m->steps_done, lr_final == lr ? 0.f : (float)epochs * m->graph_steps, lr_final};
+    const float sched[4] = {(float)m->steps_done, lr_final == lr ? 0.f : (float)epochs * m->graph_steps, lr_final, lr};
     CK(cudaMemcpyAsync(m->d_sched, sched, sizeof(sched), cudaMemcpyHostToDevice, m->stream));
     CK(cudaMemsetAsync(m->d_err, 0, 4, m->stream));
     uint64_t rs = seed ^ 0xa5a5a5a5ull;

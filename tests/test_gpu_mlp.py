@@ -555,3 +555,33 @@ def test_split_gemms_recover_from_waits_that_ran_out(gb):
             for a, b in zip(grads()[1:], before[1:]):
                 np.testing.assert_array_equal(a, b, err_msg=str(limit))
     assert ran_out > 0
+
+
+def test_second_training_call_takes_its_own_rate(gb):
+    """Two calls on one handle with the same batch and another rate: the second call's steps have the second rate,
+    bit for bit those of a handle whose training is set up anew between the calls."""
+    rng = np.random.default_rng(8)
+    X, Y = rng.normal(size=(96, 24)).astype(np.float32), rng.normal(size=(96, 16)).astype(np.float32)
+    out = []
+    for anew in (False, True):
+        m = gb.MLP(24, 16, width=32, n_layers=2, skip=True, seed=2)
+        m.set_data(X, Y)
+        m.train(1, batch=96, lr=1e-3, seed=1)
+        if anew:
+            m.set_loss_metric(None)
+        m.train(2, batch=96, lr=1e-5, lr_final=1e-6, seed=1)
+        if anew:
+            m.set_loss_metric(None)
+        p = m.params()
+        m.train(1, batch=96, lr=3e-2, seed=1)
+        out.append([a for q in (p, m.params()) for l in q for a in l if a is not None])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    # the second call moved the weights by its own rate: at most 2 steps of 1e-5 times Adam's largest ratio (about 10)
+    m = gb.MLP(24, 16, width=32, n_layers=2, skip=True, seed=2)
+    m.set_data(X, Y)
+    m.train(1, batch=96, lr=1e-3, seed=1)
+    p0 = m.params()
+    m.train(2, batch=96, lr=1e-5, seed=1)
+    for (W0, _), (W1, _) in zip(p0, m.params()):
+        assert 0 < np.abs(W1 - W0).max() < 2e-4

@@ -157,8 +157,9 @@ __global__ void __launch_bounds__(kDPanelThreads) k_dpanel(Dev d, int k0, int gu
 // FP64 pipe.
 // The pivot search is an argmax on the integer order of |a| (NaN counted as
 // +inf, the first row of the largest magnitude wins, as idamax); the scaling
-// takes the pivot's reciprocal (as LAPACK's dgetf2 does for pivots above the
-// underflow threshold).  Four threads a row, columns interleaved over them.
+// takes the pivot's reciprocal, or divides where the pivot is below the normal
+// range and its reciprocal may not be finite (as LAPACK's dgetf2 does).  Four
+// threads a row, columns interleaved over them.
 constexpr int kDPanClT = 512, kDPanLd = 36;  // row stride in doubles: 8 rows x 4 threads meet each bank pair twice
 constexpr int kDPanRows = 736;               // most rows of a CTA (212 KB)
 struct DPanMsg {
@@ -166,6 +167,7 @@ struct DPanMsg {
     unsigned long long key[16];
     int idx[16];
 };
+constexpr unsigned long long kMinNormal = 0x0010000000000000ull;  // key of 2^-1022
 __device__ __forceinline__ unsigned long long dabs_key(double v) {
     unsigned long long k = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
     return k > 0x7ff0000000000000ull ? 0x7ff0000000000000ull : k;  // NaN -> +inf
@@ -248,6 +250,7 @@ __global__ void __launch_bounds__(kDPanClT, 1) k_dpanel_cl(Dev d, int k0, int rp
         if (key == 0 || key >= 0x7ff0000000000000ull) sing = true;
         if (rank == 0 && t == 0) d.ipiv[k0 + j] = k0 + p;
         const double *pr = m.cand[w], inv = m.inv[w];
+        const bool tiny = key < kMinNormal;
         if (rank == 0 && wp == kDPanClT / 32 - 1) P[j * kDPanLd + lane] = pr[lane];  // row j is the pivot row now
         unsigned long long nkey = 0;
         int nrow = 0x7fffffff;
@@ -256,7 +259,8 @@ __global__ void __launch_bounds__(kDPanClT, 1) k_dpanel_cl(Dev d, int k0, int rp
             const bool on = r < cnt && g > j, sw = g == p && p != j;  // row p takes row j's place
             double *row = P + r * kDPanLd;
             const double *src = sw ? m.rowj : row;
-            const double l = on ? src[j] * inv : 0.0;
+            double l = on ? src[j] * inv : 0.0;
+            if (tiny && on) l = src[j] / pr[j];
             __syncwarp();
             if (on) {
 #pragma unroll
@@ -420,9 +424,11 @@ __global__ void __launch_bounds__(kDBackThreads, 1) k_dback(Dev d, int guard) {
             if (wp == 0) {
                 const double *y = ys + (b / C) * 5 * kDPanel + lane;
                 double x = y[0] - ((y[kDPanel] + y[2 * kDPanel]) + (y[3 * kDPanel] + y[4 * kDPanel]));
-                const double rd = lane < w ? 1.0 / U[lane][lane] : 0.0;
+                const double ud = lane < w ? U[lane][lane] : 1.0, rd = 1.0 / ud;
+                // (reciprocals may not be finite below the normal range: divide)
+                const bool tiny = __any_sync(0xffffffffu, dabs_key(ud) < kMinNormal);
                 for (int u = w - 1; u >= 0; u--) {
-                    if (lane == u) x *= rd;
+                    if (lane == u) x = tiny ? x / ud : x * rd;
                     const double xu = __shfl_sync(0xffffffffu, x, u);
                     if (lane < u) x = __fma_rn(-U[lane][u], xu, x);
                 }

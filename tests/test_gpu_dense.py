@@ -134,3 +134,23 @@ def test_dense_equals_sparse_at_panel_edges(gb, nbus):
     assert a["converged"] and b["converged"] and a["iterations"] == b["iterations"]
     for k in ("V", "theta"):
         np.testing.assert_allclose(a[k], b[k], rtol=0, atol=1e-11, err_msg=k)
+
+
+def test_dense_pivots_below_the_normal_range(gb):
+    """Voltages of 2^-515: the Jacobian's theta columns are subnormal, and a pivot's reciprocal is not finite.  The
+    problem scales (powers by 2^-1030, exactly but for the 44 bits that are left of the loads), so one Newton step ends
+    on the angles of the same grid at voltages of 1, and on its voltages times 2^-515."""
+    V, p = 2.0 ** -515, 2.0 ** -515 * 2.0 ** -515
+    base = np.array([0.0, 0.03, 0.05, 0.04, 0.06])
+    out = []
+    for v, q in ((1.0, 1.0), (V, p)):
+        g = gb.create_grid(bus_type=[3, 0, 0, 0, 0], V0=[v] * 5, theta0=[0.0] * 5, from_bus=[1, 2, 3, 4, 1],
+                           to_bus=[2, 3, 4, 5, 5], r=[0.02, 0.01, 0.03, 0.02, 0.04], x=[0.2, 0.15, 0.3, 0.25, 0.2])
+        s = gb.Solver(g, tolerancia=5e-324, no_max_iter=1, lim_inj_reat=0, metodo=DENSO)
+        s.set_start(V0=np.full(5, v), theta0=np.zeros(5), Pliq=-base * q, Qliq=-0.5 * base * q)
+        r = s.solve()
+        assert r["iterations"] == 1, r["status"]
+        out.append((r["theta"], r["V"] / v))
+    for a, b in zip(*out):
+        assert np.isfinite(b).all() and np.abs(a).max() > 1e-3
+        np.testing.assert_allclose(b, a, rtol=0, atol=1e-10)

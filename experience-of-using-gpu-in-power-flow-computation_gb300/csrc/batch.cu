@@ -2795,10 +2795,12 @@ struct gbpf_batch {
     // memory (layout gs = 1 or 2, the latter also compiled for four blocks
     // per SM: level 3) where that fits more instances per SM or moves factors
     // into shared memory; 2, 3, 4 take level 1, 2, 3 wherever it fits; 0
-    // never.
+    // never; spread = 1, until a plan is set: at most as many warps to a block
+    // as spread the batch over the SMs.
     struct Plan {
         int warp_mode = 1, warp_warps = 8, handoff_it = kHandoffIt, resume_group = 1, warp_group = 1, narrow = 0,
-            lu1 = 1, warp_lu1 = 0, flat_shared = 1, rotate = 0, gstate = 1, warp_gstate = 1, quad = 1;
+            lu1 = 1, warp_lu1 = 0, flat_shared = 1, rotate = 0, gstate = 1, warp_gstate = 1, quad = 1,
+            spread = 1;
     } plan;
     int block_gs = 0;  // placement level of the block-mode launch's state (layout gs)
     int warp_gs = 0;   // ... and of the warp launch's
@@ -3614,7 +3616,7 @@ gbpf_status gbpf_batch::build_graph() {
     // instances of a 118-bus grid: FP32 level 0 8 warps per SM, warp kernel
     // 8.14 ms; level 2 16 warps per SM, 6.65 ms; FP64 level 0 7 warps per SM
     // 25.3 ms, level 2 8 warps per SM 25.8 ms.  A batch that does not fill the
-    // SMs spreads over all of them, as few warps to a block as that takes, with
+    // SMs spreads over all of them (plan.spread), as few warps to a block as that takes, with
     // its state in shared memory: a warp is a serial chain, and eight on one SM
     // share its FP64 pipes while other SMs idle (300 instances on eight warps a
     // block and on two: 14 buses FP32 0.077 -> 0.064 ms, 57 buses 0.276 ->
@@ -3638,7 +3640,7 @@ gbpf_status gbpf_batch::build_graph() {
             }
             wp.warps = (int)std::max<size_t>(1, std::min<size_t>(kWarpsMax, (size_t)maxsm / wp.slice));
             if (plan.warp_warps > 0) wp.warps = std::min(wp.warps, plan.warp_warps);
-            wp.warps = std::min(wp.warps, per_sm_w);
+            if (plan.spread) wp.warps = std::min(wp.warps, per_sm_w);
             const size_t sm = (size_t)wp.warps * wp.slice;
             const void *fn = fp32 ? warp_kernel<float>(gs) : warp_kernel<double>(gs);
             if (const gbpf_status st = opt_in_smem(fn, device)) return st;
@@ -3653,7 +3655,7 @@ gbpf_status gbpf_batch::build_graph() {
                 WarpPlan c;
                 if ((wst = plan_warps(gs, c)) != GBPF_OK) return wst;
                 const bool take = plan.warp_gstate >= 2 ? (gs == plan.warp_gstate - 1 && c.occ > 0)
-                                                        : wp.occ * wp.warps < per_sm_w &&
+                                                        : !(plan.spread && wp.occ * wp.warps >= per_sm_w) &&
                                                               2 * c.occ * c.warps >= 3 * wp.occ * wp.warps;
                 if (take) {
                     wp = c;
@@ -4054,6 +4056,7 @@ extern "C" gbpf_status gbpf_batch_set_plan(gbpf_batch *b, const int plan[12]) {
     CK(cudaSetDevice(b->device));
     b->plan.warp_mode = plan[0];
     b->plan.warp_warps = plan[1];
+    b->plan.spread = 0;
     b->plan.handoff_it = plan[2];
     b->plan.resume_group = plan[3];
     b->plan.warp_group = plan[4];

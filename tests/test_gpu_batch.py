@@ -639,3 +639,25 @@ def test_small_batches_in_flight_share_the_gpu(gb, name, prec, n):
     for b, a in zip(bs, alone):
         np.testing.assert_array_equal(b.results()["V"], a["V"])
     assert four < 2.0 * one, (one, four)
+
+
+def test_batch_plan_in_warps_per_block_is_obeyed(gb):
+    """A batch of fewer instances than the plan's warps would fill spreads over the SMs by itself; a plan that was set
+    gives its warps to a block all the same, with the same bits."""
+    grid = gb.generate(4, 5, nbus=30)
+    sms = int(gb.device_info()["props"][5])
+    n = 2 * sms
+    lf = np.random.default_rng(3).uniform(0.9, 1.1, (n, grid.nB))
+    Pl = (grid.buses()["Pload"] * lf).ravel()
+    ref = None
+    for plan, used in ((None, 2), (8, 8), (3, 3), (1, 1), (0, 16)):
+        b = gb.Batch([grid], precision=gb.PREC_FP32_IR, tolerancia=1e-8, no_max_iter=30, lim_inj_reat=0)
+        if plan is not None:
+            b.set_plan(warps_per_block=plan)
+        b.set_instances(np.zeros(n, np.int32), Pload=Pl)
+        b.solve()
+        r = b.results()
+        assert b.plan()["warps_per_block_used"] == used
+        ref = ref or r
+        for k in ("iterations", "V", "theta"):
+            np.testing.assert_array_equal(r[k], ref[k], err_msg=k)

@@ -1644,7 +1644,11 @@ extern "C" gbpf_status gbpf_solver_profile(gbpf_solver *s, int repeats, double m
         else s->launch_backward(0);
     };
     CK(cudaMemsetAsync(&s->d.ctl->done, 0, sizeof(int), s->stream));
+    // (both substitutions run in the factorisation's launch: no fourth phase)
+    const bool fused = !dense && s->lu_fused;
     for (int ph = 0; ph < 4; ph++) {
+        ms[ph] = 0;
+        if (ph == 3 && fused) break;
         phase(ph);  // warm-up
         CK(cudaEventRecord(s->ev0, s->stream));
         for (int r = 0; r < repeats; r++) phase(ph);
@@ -1678,6 +1682,10 @@ extern "C" gbpf_status gbpf_solver_profile(gbpf_solver *s, int repeats, double m
     bytes[2] = 2 * b4 * nq + b4 * n + 4 * (n + 1) + 8 * nup + 4 * (nup + 1) + 8 * (nup + 1) + 8 * np + (16 + b2) * n + 4 * n;
     // backward: U blocks, inverses, columns, y in, x out
     bytes[3] = b4 * nup + b4 * n + 4 * (n + 1) + 4 * nup + 2 * b2 * n + 4 * n;
+    if (fused) {
+        bytes[2] += bytes[3];
+        bytes[3] = 0;
+    }
     return GBPF_OK;
 }
 

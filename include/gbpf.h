@@ -357,9 +357,12 @@ gbpf_status gbpf_solver_setup_times(const gbpf_solver *s, double ms[5]);
  * last solve's state left on the device, `repeats` passes after one warm-up):
  * [0] injections + limits + mismatch, [1] Jacobian fill, [2] LU
  * factorisation fused with forward substitution (all levels), [3] backward
- * substitution (all levels); with metodo = denso [1] the dense fill, [2] the
- * blocked LU, [3] the triangular solves.  bytes[] = algorithmic bytes of one
- * pass (in the factor's precision). */
+ * substitution (all levels) where it is launched by itself; where one launch
+ * takes the LU and both substitutions (gbpf_solver_set_lu_launch modes 0 and
+ * 2) they are all in [2], and [3] is 0.  With metodo = denso [1] the dense
+ * fill, [2] the blocked LU, which takes the right-hand side through the
+ * forward substitution, [3] the backward substitution.  bytes[] = algorithmic
+ * bytes of one pass (in the factor's precision). */
 gbpf_status gbpf_solver_profile(gbpf_solver *s, int repeats, double ms[4], long long bytes[4]);
 
 /* ------------------------------------------------------------------------ */

@@ -107,3 +107,21 @@ def test_results_come_back_in_one_piece(gb, name, max_iter):
             assert getattr(gb.lib(), call)(s.h, *ptr) == 0
             for i, k in enumerate(keys):
                 np.testing.assert_array_equal(a[i], r[k] if mask >> i & 1 else np.full(n, np.nan), err_msg=k)
+
+
+@pytest.mark.parametrize("precision", ["PREC_FP64", "PREC_FP32_IR"])
+def test_profile_counts_the_substitutions_where_they_run(gb, precision):
+    """The backward substitution is a phase of its own only where it is launched by itself: in the forms that take it
+    with the factorisation its time and bytes are zero and its bytes are the factorisation's."""
+    s = gb.Solver(grid_of(gb, "c5_base.cdf.gz"), tolerancia=1e-8, no_max_iter=100, metodo=0, precision=getattr(gb, precision))
+    s.set_form(gb.FORM_GRAPH)
+    s.solve(full=False)
+    p = {}
+    for mode in (0, 1, 2):
+        s.set_lu_launch(mode)
+        p[mode] = s.profile(3)
+    assert p[1]["backward"]["ms"] > 0 and p[1]["backward"]["bytes"] > 0
+    for mode in (0, 2):
+        assert p[mode]["backward"] == dict(ms=0.0, bytes=0)
+        assert p[mode]["factor_forward"]["ms"] > 0
+        assert p[mode]["factor_forward"]["bytes"] == p[1]["factor_forward"]["bytes"] + p[1]["backward"]["bytes"]

@@ -884,10 +884,10 @@ struct gbpf_solver {
     size_t cl_smem = 0;
     void *cl_mem = nullptr;  // the schedule
     gbpf_status plan_cluster();
-    cudaLaunchConfig_t cluster_config(int ctas, size_t smem, cudaLaunchAttribute *at) const {
+    cudaLaunchConfig_t cluster_config(int ctas, int threads, size_t smem, cudaLaunchAttribute *at) const {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(ctas);
-        cfg.blockDim = dim3(kClT);
+        cfg.blockDim = dim3(threads);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream;
         at->id = cudaLaunchAttributeClusterDimension;
@@ -896,6 +896,24 @@ struct gbpf_solver {
         cfg.attrs = at;
         cfg.numAttrs = 1;
         return cfg;
+    }
+    // A cluster that the device does not take is refused at the launch, while
+    // the graph is captured as well: launched() is asked before a graph is
+    // instantiated or results are read.
+    cudaError_t launch_err = cudaSuccess;
+    template <class... P, class... A>
+    void launch_cluster(void (*fn)(P...), int ctas, int threads, size_t smem, A... args) {
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = cluster_config(ctas, threads, smem, at);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, args...);
+        if (e != cudaSuccess) launch_err = e;
+    }
+    gbpf_status launched() {
+        const cudaError_t l = cudaGetLastError(), e = launch_err ? launch_err : l;
+        launch_err = cudaSuccess;
+        if (e == cudaSuccess) return GBPF_OK;
+        set_error(std::string("kernel launch: ") + cudaGetErrorString(e));
+        return GBPF_E_CUDA;
     }
     int lu_mode(int mode) const {
         if (mode == 0 && cl_ctas && !(d.fp32 && opt.lim_inj_reat && S.n <= kFusedMaxN32)) return 2;
@@ -908,9 +926,7 @@ struct gbpf_solver {
             return;
         }
         if (lu_fused == 2) {
-            cudaLaunchAttribute at[1];
-            const cudaLaunchConfig_t cfg = cluster_config(cl_ctas, cl_smem, at);
-            (void)cudaLaunchKernelEx(&cfg, k_lu_cluster<TJ>, d, cl_args, guard);
+            launch_cluster(k_lu_cluster<TJ>, cl_ctas, kClT, cl_smem, d, cl_args, guard);
             return;
         }
         for (int l = 0; l < nfl(); l++) {
@@ -954,29 +970,22 @@ struct gbpf_solver {
     }
     void launch_dense_lu(int guard) {
         const int N = d.N;
-        cudaLaunchAttribute at[1];
         for (int k0 = 0; k0 < N; k0 += kDPanel) {
             const int nb = std::min(kDPanel, N - k0), k1 = k0 + nb, R = N - k0;
             // rows of a CTA: an even share, no fewer than the panel's columns
             const int rp = std::max(kDPanel, cdiv_int(R, kDCtas));
             int ctas = 1;
             while (ctas * rp < R) ctas *= 2;
-            if (rp <= kDPanRows) {
-                cudaLaunchConfig_t cfg = cluster_config(ctas, sizeof(double) * (size_t)rp * kDPanLd, at);
-                cfg.blockDim = dim3(kDPanClT);
-                (void)cudaLaunchKernelEx(&cfg, k_dpanel_cl, d, k0, rp, guard);
-            } else {
+            if (rp <= kDPanRows)
+                launch_cluster(k_dpanel_cl, ctas, kDPanClT, sizeof(double) * (size_t)rp * kDPanLd, d, k0, rp, guard);
+            else
                 k_dpanel<<<1, kDPanelThreads, 0, stream>>>(d, k0, guard);
-            }
             k_dswap<<<cdiv_int(N + 1 - nb, 8), 256, 0, stream>>>(d, k0, guard);
             if (k1 < N) k_dgemm<<<dim3(cdiv_int(N + 1 - k1, 32), cdiv_int(N - k1, 64)), 256, 0, stream>>>(d, k0, guard);
         }
     }
     void launch_dense_solve(int guard) {
-        cudaLaunchAttribute at[1];
-        cudaLaunchConfig_t cfg = cluster_config(kDCtas, dense_back_smem(d.N), at);
-        cfg.blockDim = dim3(kDBackThreads);
-        (void)cudaLaunchKernelEx(&cfg, k_dback, d, guard);
+        launch_cluster(k_dback, kDCtas, kDBackThreads, dense_back_smem(d.N), d, guard);
     }
     static size_t dense_back_smem(int N) {
         return sizeof(double) * 5 * kDPanel * (size_t)cdiv_int(cdiv_int(N, kDPanel), kDCtas);
@@ -1245,7 +1254,7 @@ gbpf_status gbpf_solver::plan_cluster() {
                      at_sched = at_tail + cl.tail_bytes, sm = at_sched + cl.sched_bytes;
         CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
         cudaLaunchAttribute at[1];
-        const cudaLaunchConfig_t cfg = cluster_config(cl.ctas, sm, at);
+        const cudaLaunchConfig_t cfg = cluster_config(cl.ctas, kClT, sm, at);
         int fit = 0;
         if (cudaOccupancyMaxActiveClusters(&fit, fn, &cfg) != cudaSuccess) { (void)cudaGetLastError(); fit = 0; }
         if (fit < 1) continue;
@@ -1326,6 +1335,7 @@ gbpf_status gbpf_solver::build_graph() {
         // (one limit for all solvers: the largest system's)
         CK(cudaFuncSetAttribute(k_dback, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dense_back_smem(kDenseMaxN)));
     }
+    (void)cudaGetLastError();  // what launched() finds is of this graph
     CK(cudaGraphCreate(&graph, 0));
     cudaGraphConditionalHandle h;
     CK(cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault));
@@ -1361,6 +1371,11 @@ gbpf_status gbpf_solver::build_graph() {
     CK(cudaStreamBeginCaptureToGraph(stream, graph, &wnode, nullptr, 1, cudaStreamCaptureModeThreadLocal));
     if (g.nL) k_flows<<<cdiv_int(g.nL, T), T, 0, stream>>>(d);
     CK(cudaStreamEndCapture(stream, &g2));
+    if (const gbpf_status st = launched()) {
+        cudaGraphDestroy(graph);
+        graph = nullptr;
+        return st;
+    }
     CK(cudaGraphInstantiate(&exec, graph, 0));
     size_t nn = 0;
     CK(cudaGraphGetNodes(graph, nullptr, &nn));
@@ -1658,7 +1673,7 @@ extern "C" gbpf_status gbpf_solver_profile(gbpf_solver *s, int repeats, double m
         CK(cudaEventElapsedTime(&t, s->ev0, s->ev1));
         ms[ph] = t / repeats;
     }
-    CK(cudaGetLastError());
+    if (const gbpf_status e = s->launched()) return e;
     const long long nB = s->g.nB, nnzY = s->y.nnz, n = S.n, nup = S.nup, np = S.pairs();
     // block and vector sizes of the factor's precision
     const long long b4 = s->d.fp32 ? 16 : 32, b2 = s->d.fp32 ? 8 : 16;
@@ -1809,7 +1824,7 @@ extern "C" gbpf_status gbpf_newton_step(gbpf_solver *s, const double *V, const d
     const int nq = S.n + 2 * S.nup, T = 256;
     k_jfill<<<cdiv_int(nq, T), T, 0, s->stream>>>(s->d, 0);
     s->launch_factor_solve(0);
-    CK(cudaGetLastError());
+    if ((st = s->launched()) != GBPF_OK) return st;
     std::vector<double2> x(S.n);
     std::vector<float2> x32(s->d.fp32 ? S.n : 0);
     Ctl c;
@@ -1970,7 +1985,7 @@ extern "C" gbpf_status gbpf_solve_traced(gbpf_solver *s, gbpf_result *r, gbpf_tr
         } else {
             s->launch_factor_solve(0);
         }
-        CK(cudaGetLastError());
+        if (const gbpf_status e = s->launched()) return e;
         if (d.fp32) {
             CK(cudaMemcpyAsync(x32.data(), d.xs32, n * sizeof(float2), D2H, st));
         } else {

@@ -125,3 +125,31 @@ def test_profile_counts_the_substitutions_where_they_run(gb, precision):
         assert p[mode]["backward"] == dict(ms=0.0, bytes=0)
         assert p[mode]["factor_forward"]["ms"] > 0
         assert p[mode]["factor_forward"]["bytes"] == p[1]["factor_forward"]["bytes"] + p[1]["backward"]["bytes"]
+
+
+# Backward error of a Newton step, |J dx - g| / (max row sum of |J| times |dx|): 1e-13 in FP64 as in the test of the
+# 236-bus grid above, and 2^29 times that in FP32.
+@pytest.mark.parametrize("precision,tol", [("PREC_FP64", 1e-13), ("PREC_FP32_IR", 1e-13 * 2 ** 29)])
+@pytest.mark.parametrize("name", ["gen944", "tiles256"])
+def test_cluster_lu_with_its_schedule_in_global_memory(gb, name, precision, tol):
+    """Schedules that no CTA's shared memory holds: a filled 944-bus grid (lists of one int a pair) and a chain of 256
+    copies of 118 buses, whose 80,375 factor blocks a triangle need lists of two ints a pair.  (That chain's Newton
+    diverges from the flat start, on the CPU as well, so it is one Newton step that is held against the Jacobian.)"""
+    sparse = pytest.importorskip("scipy.sparse")
+    grid = gb.generate(3, 1, tiles=256) if name == "tiles256" else grid_of(gb, name)
+    b = grid.buses()
+    V, th = b["V0"], b["theta0"] + 0.01 * np.sin(np.arange(grid.nB))
+    for mode in (0, 1):
+        s = gb.Solver(grid, tolerancia=1e-8, no_max_iter=100, lim_inj_reat=0, metodo=0, precision=getattr(gb, precision))
+        s.set_lu_launch(mode)
+        info = s.info()
+        assert info["factor_blocks"] > (65536 if name == "tiles256" else 16000)
+        assert (info["kernels_per_iteration"] < 12) == (mode == 0)
+        row, col, val = s.eval_jacobian(V, th)
+        n = int(row.max()) + 1
+        J = sparse.csr_matrix((val, (row, col)), shape=(n, n))
+        g = np.cos(np.arange(n))
+        dx = s.newton_step(V, th, g)
+        assert np.isfinite(dx).all()
+        assert np.abs(J @ dx - g).max() <= tol * abs(J).sum(axis=1).max() * np.abs(dx).max(), mode
+        s.close()

@@ -154,3 +154,19 @@ def test_dense_pivots_below_the_normal_range(gb):
     for a, b in zip(*out):
         assert np.isfinite(b).all() and np.abs(a).max() > 1e-3
         np.testing.assert_allclose(b, a, rtol=0, atol=1e-10)
+
+
+def test_dense_panels_too_tall_for_a_cluster(gb):
+    """5,900 buses, N = 11,798: the first panel has more rows than sixteen CTAs hold and is factored on one block
+    (k_dpanel), the others on clusters.  Newton from the flat start, held against the sparse form to 1e-9."""
+    grid = gb.generate(3, 1, tiles=50)
+    assert 2 * (grid.nB - 1) > 16 * 736
+    out = []
+    for metodo in (DENSO, 0):
+        s = gb.Solver(grid, tolerancia=1e-8, no_max_iter=20, lim_inj_reat=0, metodo=metodo)
+        out.append(s.solve())
+        s.close()
+    a, b = out
+    assert a["converged"] and b["converged"] and a["iterations"] == b["iterations"]
+    for k in ("V", "theta"):
+        np.testing.assert_allclose(a[k], b[k], rtol=0, atol=STATE_TOL, err_msg=k)

@@ -661,3 +661,42 @@ def test_batch_plan_in_warps_per_block_is_obeyed(gb):
         ref = ref or r
         for k in ("iterations", "V", "theta"):
             np.testing.assert_array_equal(r[k], ref[k], err_msg=k)
+
+
+@pytest.mark.parametrize("nbus", [14, 57, 97, 118])
+def test_batch_fp32_warp_records_keep_the_lists_bits(gb, nbus):
+    """Iteration 0 of an FP32 batch on warps once from its topology's shared copy, whose factor comes from the levels'
+    lists, and once by each warp itself, from the records of its lanes: the same bits, at the end as well."""
+    grid = gb.generate(4, 7, nbus=nbus)
+    base, n = grid.buses(), 40
+    lf = np.random.default_rng(nbus).uniform(0.9, 1.1, (n, grid.nB))
+    out = []
+    for shared in (1, 0):
+        b = gb.Batch([grid], precision=gb.PREC_FP32_IR, tolerancia=1e-8, no_max_iter=30, lim_inj_reat=0)
+        b.set_plan(flat_shared=shared, handoff_it=0)
+        b.set_instances(np.zeros(n, np.int32), Pload=(base["Pload"] * lf).ravel(), Qload=(base["Qload"] * lf).ravel())
+        b.solve()
+        assert b.plan()["warp_instances"] == n
+        out.append(b.results())
+    for k in ("iterations", "status", "V", "theta"):
+        np.testing.assert_array_equal(out[0][k], out[1][k], err_msg=k)
+
+
+def test_batch_fp32_block_records_keep_the_lists_bits(gb):
+    """The forward levels of FP32 instances on blocks from records (two blocks per SM) and from the lists (four): the
+    same bits."""
+    import bench
+
+    grid = gb.read_grid(bench.grid_file("c5_base.cdf.gz"))
+    base, n = grid.buses(), 12
+    lf = np.random.default_rng(5).uniform(0.95, 1.05, (n, grid.nB))
+    out = []
+    for gs in (3, 4):
+        b = gb.Batch([grid], precision=gb.PREC_FP32_IR, tolerancia=1e-8, no_max_iter=30, lim_inj_reat=0)
+        b.set_plan(gstate=gs)
+        b.set_instances(np.zeros(n, np.int32), Pload=(base["Pload"] * lf).ravel(), Qload=(base["Qload"] * lf).ravel())
+        b.solve()
+        assert b.plan()["block_instances"] == n and b.plan()["block_state_global"] == gs - 1
+        out.append(b.results())
+    for k in ("iterations", "status", "V", "theta"):
+        np.testing.assert_array_equal(out[0][k], out[1][k], err_msg=k)

@@ -425,13 +425,16 @@ __global__ void __launch_bounds__(kDBackThreads, 1) k_dback(Dev d, int guard) {
                 const double *y = ys + (b / C) * 5 * kDPanel + lane;
                 double x = y[0] - ((y[kDPanel] + y[2 * kDPanel]) + (y[3 * kDPanel] + y[4 * kDPanel]));
                 const double ud = lane < w ? U[lane][lane] : 1.0, rd = 1.0 / ud;
+                auto rows = [&](auto over) {
+                    for (int u = w - 1; u >= 0; u--) {
+                        if (lane == u) x = over(x);
+                        const double xu = __shfl_sync(0xffffffffu, x, u);
+                        if (lane < u) x = __fma_rn(-U[lane][u], xu, x);
+                    }
+                };
                 // (reciprocals may not be finite below the normal range: divide)
-                const bool tiny = __any_sync(0xffffffffu, dabs_key(ud) < kMinNormal);
-                for (int u = w - 1; u >= 0; u--) {
-                    if (lane == u) x = tiny ? x / ud : x * rd;
-                    const double xu = __shfl_sync(0xffffffffu, x, u);
-                    if (lane < u) x = __fma_rn(-U[lane][u], xu, x);
-                }
+                if (__any_sync(0xffffffffu, dabs_key(ud) < kMinNormal)) rows([&](double v) { return v / ud; });
+                else rows([&](double v) { return v * rd; });
                 for (int q = 0; q < C; q++) cl_put(cl_map(&xb[b & 1][lane], q), x);
                 if (lane < w) ((double *)d.xs)[r0 + lane] = x;
             }

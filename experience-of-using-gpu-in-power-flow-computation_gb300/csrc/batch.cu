@@ -727,10 +727,10 @@ __device__ __forceinline__ void back_rows(const TopoView &G, int l, int lg, int 
 // than the block takes at a time), laid out by thread by add_topology: a level
 // begins behind a barrier, and there its lists were a chain of four loads (the
 // level's step, the range of its list, the list, the blocks); a record is one,
-// made a round ahead (150 FP32 instances of a 1,888-bus grid 0.92 -> 0.79 ms,
-// 250 of 236 buses 0.39 -> 0.34).  At four blocks per SM the other blocks fill
-// the waits and the records' own traffic costs more: there the forward levels
-// keep their lists (2,048 instances of 1,888 buses 6.08 ms, with records 6.30).
+// made a round ahead (250 FP32 instances of a filled 236-bus grid 0.39 -> 0.34
+// ms).  At four blocks per SM the other blocks fill the waits and the records'
+// own traffic costs more: there the forward levels keep their lists (2,048
+// instances of 1,888 buses 6.08 ms, with records 6.30).
 struct LuRec {
     const int4 *piv;   // step (-1: none), first and last + 1 of its list for this lane, position of the first
     const int *pk;     // step of that position
@@ -1809,7 +1809,7 @@ __global__ void __launch_bounds__(kThreads, GS == 3 ? 4 : 2) k_nr_block(Args a) 
                     // Jacobian fill at every factor position (zeros at fill-in)
                     // (two at a time, as the other loops over buses here: loads that do
                     // not wait for a store go out together; 2,048 FP32 instances of a
-                    // 1,888-bus grid 5.88 -> 5.57 ms, 150 of them 0.79 -> 0.69)
+                    // 1,888-bus grid 5.88 -> 5.57 ms)
                     for (int q = tid; q < nq; q += 2 * kThreads) {
                         const int q1 = min(q + kThreads, nq - 1);
                         const B4 b0 = jac_block<TJ>(G, q, n, act, P, Q, V, cs, sn, f32);
@@ -3619,8 +3619,8 @@ gbpf_status gbpf_batch::build_graph() {
     // SMs spreads over all of them (plan.spread), as few warps to a block as that takes, with
     // its state in shared memory: a warp is a serial chain, and eight on one SM
     // share its FP64 pipes while other SMs idle (300 instances on eight warps a
-    // block and on two: 14 buses FP32 0.077 -> 0.064 ms, 57 buses 0.276 ->
-    // 0.166, 118 buses 0.327 -> 0.203, FP64 0.526 -> 0.384; the lines meet at
+    // block and on two: 14 buses FP32 0.066 -> 0.055 ms, 57 buses 0.215 ->
+    // 0.178, 118 buses 0.258 -> 0.215, FP64 0.522 -> 0.394; the lines meet at
     // eight warps per SM, 1,216 instances).
     warp_grid = 0;
     warp_gs = 0;

@@ -647,14 +647,15 @@ __global__ void k_bsolve(Dev d, int beg, int cnt, int guard) {
 // next level boundary, as the per-level launches stop (guard).
 constexpr int kFusedThreads = 512;
 // Largest Jacobian block order that takes k_lu_fused rather than a launch per
-// level where k_lu_cluster does not run: FP32 with reactive limits (the limit
-// check looks at the size of the Newton step, whose FP32 rounding k_lu_fused's
-// order of sums keeps on the FP64 switch path of the 118-bus golden cases),
-// and GPUs without clusters of 8.  Measured on single solves (ms per solve,
-// per-level launches -> k_lu_fused): FP32 57 buses 0.99 -> 0.57, 118 0.79 ->
-// 0.46, 236 5.7 -> 3.5, 472 18.5 -> 13.3, 944 19.8 -> 23.3, 1,888 1.35 -> 1.73;
-// FP64 57 1.99 -> 1.76, 118 1.53 -> 1.40, 236 16.9 -> 19.6 (one SM's FP64 pipe
-// is too small for more).
+// level where k_lu_cluster does not run: FP32 with reactive limits, and GPUs
+// without clusters of 8.  (The limit check looks at the size of the Newton
+// step, and another order of its FP32 sums can switch other PV buses, on the
+// 118-bus golden cases to begin with; grids of this size keep the order they
+// were solved with, though the cluster is faster on the larger of them.)
+// Measured on single solves (ms per solve, per-level launches -> k_lu_fused):
+// FP32 57 buses 0.99 -> 0.57, 118 0.79 -> 0.46, 236 5.7 -> 3.5, 472 18.5 ->
+// 13.3, 944 19.8 -> 23.3, 1,888 1.35 -> 1.73; FP64 57 1.99 -> 1.76, 118 1.53
+// -> 1.40, 236 16.9 -> 19.6 (one SM's FP64 pipe is too small for more).
 constexpr int kFusedMaxN32 = 600, kFusedMaxN64 = 150;
 // Largest factor (off-diagonal blocks a triangle) whose FP64 solve takes the
 // persistent form by default (see gbpf_solver::build).

@@ -455,6 +455,10 @@ struct ClusterBuilder {
         const ClusterSplit L = split(t0);
         const size_t per = S.nup <= 65536 && n <= 65536 ? 4 : 8;
         double items0 = 0, pairs0 = 0;  // of CTA 0
+        // what a level takes besides its work: on the cluster a store, a cluster
+        // barrier and a load from L2 (2,650 cycles measured; the barrier alone 380
+        // to 480, with the store 1,760), in the segment two block barriers and the
+        // loads between them
         const double clus = 3000, seg = 400;
         auto fwd = [&](const std::vector<int> &steps, bool in_seg, int share) {
             long long md = 0, sd = 0, ne = 0, me = 0, se = 0;

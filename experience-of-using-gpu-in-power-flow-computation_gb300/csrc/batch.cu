@@ -2804,6 +2804,7 @@ struct gbpf_batch {
     } plan;
     int block_gs = 0;  // placement level of the block-mode launch's state (layout gs)
     int warp_gs = 0;   // ... and of the warp launch's
+    int block_carve = -1, warp_carve = -1;  // division of L1 and shared memory that they ask for
     DevBuf gstate_mem, warp_gstate_mem;
     gbpf_status rebuild() {
         CK(cudaStreamSynchronize(stream));
@@ -3355,9 +3356,21 @@ gbpf_status gbpf_batch::set_instances(int n, const int *tofi, const double *Ploa
 
 gbpf_status gbpf_batch::launch(cudaStream_t st) { return launch_with(st, args, wargs, true); }
 
-static void launch_kernel(const void *fn, int grid, int threads, size_t smem, cudaStream_t st, const Args &a) {
+// carve: share of the SM's L1 and shared memory, in percent, that the launch
+// asks for as shared memory (-1: the driver's choice)
+static void launch_kernel(const void *fn, int grid, int threads, size_t smem, cudaStream_t st, const Args &a, int carve) {
+    cudaLaunchConfig_t c{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at.val.sharedMemCarveout = (unsigned)carve;
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = carve >= 0;
     void *args[] = {(void *)&a};
-    (void)cudaLaunchKernel(fn, dim3(grid), dim3(threads), args, smem, st);
+    (void)cudaLaunchKernelExC(&c, fn, args);
 }
 
 // One persistent launch per mode over the queues of ba (blocks) and wa (warps).
@@ -3369,7 +3382,7 @@ gbpf_status gbpf_batch::launch_with(cudaStream_t st, const Args &ba, const Args 
         CK(cudaStreamWaitEvent(side, fork, 0));
         if (timed) CK(cudaEventRecordWithFlags(kev[0], side, cudaEventRecordExternal));
         launch_kernel(fp32 ? blk_kernel<float>(block_gs) : blk_kernel<double>(block_gs), grid_blocks, kThreads, smem, side,
-                      ba);
+                      ba, block_carve);
         {
             const cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) {
@@ -3388,7 +3401,7 @@ gbpf_status gbpf_batch::launch_with(cudaStream_t st, const Args &ba, const Args 
     if (wa.queue_len) {
         if (timed) CK(cudaEventRecordWithFlags(kev[2], st, cudaEventRecordExternal));
         launch_kernel(fp32 ? warp_kernel<float>(warp_gs) : warp_kernel<double>(warp_gs), warp_grid, 32 * warp_warps,
-                      warp_smem, st, wa);
+                      warp_smem, st, wa, warp_carve);
         CK_LAUNCH();
         if (timed) CK(cudaEventRecordWithFlags(kev[3], st, cudaEventRecordExternal));
         if (wa.handoff_it > 0) {
@@ -3450,6 +3463,21 @@ gbpf_status gbpf_batch::build_graph() {
     CK(cudaMalloc(&queues.p, 4 * (size_t)n_inst + 256));
     if (n_warp_q) CK(cudaMemcpy(queues.p, wq.data(), 4 * wq.size(), cudaMemcpyHostToDevice));
     if (n_block_q) CK(cudaMemcpy((int *)queues.p + n_warp_q, bq.data(), 4 * bq.size(), cudaMemcpyHostToDevice));
+    // A launch whose own blocks fill every SM asks for the shared memory of those
+    // and no more: the rest is L1, where the index lists and global factors are
+    // read from (2,048 FP32 instances of a 1,888-bus grid 4.57 -> 4.50 ms; 608 of
+    // them behind 100 of 118 buses 1.80 -> 1.50).  A smaller one leaves the
+    // division to the driver: asked for exactly, it keeps the blocks of other
+    // batches in flight from the SMs (four batches of 300 FP32 instances of 57
+    // buses 0.21 -> 0.54 ms).
+    int sm_smem = 0;
+    CK(cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
+    auto carve_of = [&](int grid, int occ, int work, size_t dyn) {  // occ blocks of dyn bytes and static and reserved ones
+        if (occ < 1 || grid < dev_sm * occ || work < grid) return -1;
+        const size_t want = 100 * (size_t)occ * (dyn + 1280);
+        return (int)std::min<size_t>(100, (want + sm_smem - 1) / sm_smem);
+    };
+    block_carve = warp_carve = -1;
     // Block-mode shared-memory plan: the blob is staged in shared memory when
     // at most 48 KB; the factor stays in shared memory when blob region +
     // state + factor fit in 110 KB, otherwise it lives in global scratch.
@@ -3458,10 +3486,9 @@ gbpf_status gbpf_batch::build_graph() {
     // SM, or as many with more factors and tails in shared memory.  A tail has
     // its place before the factor.  The plan looks at the grids alone and not
     // at the number of instances: other batches may be in flight beside this
-    // one, on their own streams, and a plan (or a division of L1 and shared
-    // memory asked for at the launch) that gives a small batch all of an SM
-    // makes them wait for one another.  Four batches of 100 FP32 instances of a
-    // 1,888-bus grid launched together: 1.78 ms with the whole SM planned for
+    // one, on their own streams, and a plan that gives a small batch all of an
+    // SM makes them wait for one another.  Four batches of 100 FP32 instances of
+    // a 1,888-bus grid launched together: 1.78 ms with the whole SM planned for
     // one, 1.07 as it is (alone 0.55 and 0.71).
     const size_t budget = 110 * 1024, blob_cap = 48 * 1024;
     size_t region = 0;
@@ -3596,6 +3623,7 @@ gbpf_status gbpf_batch::build_graph() {
         int occ = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, blk_fn(block_gs), kThreads, smem));
         grid_blocks = std::max(1, std::min(n_block_q, dev_sm * std::max(occ, 1)));
+        if (!n_warp_q) block_carve = carve_of(grid_blocks, occ, n_block_q, smem);
     }
     if (use_handoff) {
         int occ = 0;
@@ -3667,6 +3695,7 @@ gbpf_status gbpf_batch::build_graph() {
         warp_warps = wp.warps;
         warp_smem = (size_t)warp_warps * slice;
         warp_grid = std::max(1, std::min((n_warp_q + warp_warps - 1) / warp_warps, dev_sm * std::max(wp.occ, 1)));
+        if (!n_block_q) warp_carve = carve_of(warp_grid, wp.occ, n_warp_q, warp_smem);
         warp_gstride = warp_gs ? align_up(wp.gst, 256) : 0;
     }
     warp_gstate_mem.reset();
